@@ -125,11 +125,11 @@ __global__ void __launch_bounds__(256) k_diffusion_bwd(const float* __restrict__
 
 // Gather RB rows of a kx-major spectrum (src[kx * N + s]) into the row
 // buffer (transposed) with per-element async copies; waits for them.
-template <int LOGN, int V = 0>
-__device__ __forceinline__ void gather_rows(const float2* __restrict__ src, float2* buf) {
-    using G = Geo<LOGN, V>;
-    for_row_tile<LOGN, V>([&](int s, int kx, int pk) {
-        cp_async8(&buf[s * G::RP + pk], &src[size_t(kx) * G::N + s]);
+template <class G, class ROW = RowsInOrder>
+__device__ __forceinline__ void gather_rows(const float2* __restrict__ src, float2* buf,
+                                            ROW row = ROW()) {
+    for_row_tile<G>([&](int s, int kx, int pk) {
+        cp_async8(&buf[s * G::RP + pk], &src[size_t(kx) * G::N + row(s)]);
     });
     cp_async_commit();
     cp_async_wait<0>();
@@ -138,9 +138,8 @@ __device__ __forceinline__ void gather_rows(const float2* __restrict__ src, floa
 
 // Inverse row FFT of RB packed rows in `buf`; `out(s, i, v)` receives the
 // pixel pair (x[2i], x[2i+1]) of row s.
-template <int LOGN, int V, class OUT>
+template <class G, class OUT>
 __device__ __forceinline__ void c2r_rows(float2* buf, const float2* __restrict__ tw, OUT& out) {
-    using G = Geo<LOGN, V>;
     SmemRows rows{buf, G::RP};
     // m = j + q (M / R): m = 0 only in slot q = 0 (compile-time)
     auto ld0 = [&](int s, int m, int, int q) -> float2 {
@@ -175,21 +174,56 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // 3. Growth backward, one kernel's RB rows per CTA (RT threads):
 //    U[k] rows -> u -> ubar -> forward row FFT -> written over U[k].
 // ---------------------------------------------------------------------------
+// The rows of a CTA.  A thread adds its values to three FP32 sums before the
+// block adds the threads' sums in FP64, so which values share a thread decides
+// the parameter gradients' rounding.  At sides 64 to 256 a thread sums CHAIN
+// rows `stride` apart (32 where the world runs untuned, 8 where variants were
+// chosen), whatever the CTA shape: CTAs of 64 threads take 4 adjacent rows
+// of each of the CHAIN groups.  Elsewhere a thread's rows follow from the shape
+// (at 16, 32 and 512 a thread has one row's 16 values in every shape).
+template <int LOGN, int V, bool CHAINED = (LOGN >= 6 && LOGN <= 8)>
+struct GrowthRows : Geo<LOGN, V> {
+    static constexpr int CHAIN = 1, GROUP = Geo<LOGN, V>::RB;
+};
+template <int LOGN, int V>
+struct GrowthRows<LOGN, V, true> : Geo<LOGN, V> {
+    using G = Geo<LOGN, V>;
+    static constexpr int CHAIN = LOGN == 7 ? 4 : 2, GROUP = 4;
+    static constexpr int RB = GROUP * CHAIN, RT = 64;
+    static constexpr int RP = padded_len(G::M) + (RB >= 16 ? 1 : 2);
+    static constexpr size_t R2C_SMEM = size_t(RB) * RP * sizeof(float2);
+    static_assert(GROUP * (G::M / last_radix(G::M)) == RT, "one group of rows per sweep");
+};
+struct ChainedRows {
+    int group, stride;
+    __device__ __forceinline__ int operator()(int s) const {
+        return s % group + s / group * stride;
+    }
+};
+
 template <int LOGN, int V = 0>
 __device__ __forceinline__ void growth_bwd_body(float2* __restrict__ U,
                                                 const float* __restrict__ abar,
                                                 const float2* __restrict__ tw,
-                                                const AdjointParams& ap, int k, int cout, int y0,
-                                                double* __restrict__ pgrad, int K, float2* sm,
-                                                double* red) {
-    using G = Geo<LOGN, V>;
+                                                const AdjointParams& ap, int k, int cout,
+                                                int block, int stride, double* __restrict__ pgrad,
+                                                int K, float2* sm, double* red) {
+    using G = GrowthRows<LOGN, V>;
+    constexpr bool CHAINED = G::CHAIN > 1;
+    const int groups = stride / G::GROUP;   // per chain
+    const int y0 = CHAINED ? block / groups * (stride * G::CHAIN) + block % groups * G::GROUP
+                           : block * G::RB;
+    const std::conditional_t<CHAINED, ChainedRows, RowsInOrder> row = [&] {
+        if constexpr (CHAINED) return ChainedRows{G::GROUP, stride};
+        else return RowsInOrder{};
+    }();
     float2* Uk = U + size_t(k) * G::M * G::N + y0;
-    gather_rows<LOGN, V>(Uk, sm);
+    gather_rows<G>(Uk, sm, row);
     const float mu = ap.mu[k], w = ap.w[k], is2 = ap.inv_s2[k], is3 = ap.inv_s3[k];
     const float* ab = abar + (size_t(cout) * G::N + y0) * G::N;
     float pw = 0.f, pmu = 0.f, psg = 0.f;
     auto out = [&](int s, int i, float2 v) {
-        const float2 a = reinterpret_cast<const float2*>(ab + size_t(s) * G::N)[i];
+        const float2 a = reinterpret_cast<const float2*>(ab + size_t(row(s)) * G::N)[i];
         float ub[2];
         const float uu[2] = {v.x, v.y}, aa[2] = {a.x, a.y};
 #pragma unroll
@@ -205,10 +239,10 @@ __device__ __forceinline__ void growth_bwd_body(float2* __restrict__ U,
         }
         sm[s * G::RP + pidx(i)] = make_float2(ub[0], ub[1]);
     };
-    c2r_rows<LOGN, V>(sm, tw, out);
+    c2r_rows<G>(sm, tw, out);
     SmemRows rows{sm, G::RP};
     FftPasses<G::M, 1, false, G::RT, G::RB, false, G::ROW_MR>::run(rows, rows, rows, rows, tw + G::TW_ROW);
-    r2c_finish<LOGN, V>(sm, tw, Uk);
+    r2c_finish<G>(sm, tw, Uk, row);
     const double sw = block_sum(double(pw), red);
     const double smu = block_sum(double(pmu), red);
     const double ssg = block_sum(double(psg), red);
@@ -220,18 +254,17 @@ __device__ __forceinline__ void growth_bwd_body(float2* __restrict__ U,
 }
 
 template <int LOGN, int V = 0>
-__global__ void __launch_bounds__(Geo<LOGN, V>::RT, 512 / Geo<LOGN, V>::RT) k_growth_bwd(float2* __restrict__ U,
-                                                     const float* __restrict__ abar,
-                                                     const float2* __restrict__ tw,
-                                                     const AdjointParams* __restrict__ app,
-                                                     double* __restrict__ pgrad, int K) {
+__global__ void __launch_bounds__(GrowthRows<LOGN, V>::RT, 512 / GrowthRows<LOGN, V>::RT)
+    k_growth_bwd(float2* __restrict__ U, const float* __restrict__ abar,
+                 const float2* __restrict__ tw, const AdjointParams* __restrict__ app,
+                 double* __restrict__ pgrad, int K, int stride) {
     extern __shared__ __align__(128) float2 sm_gbwd[];
     __shared__ double red[16];
     pdl_wait();
     pdl_launch_dependents();
     const int k = blockIdx.y;
-    growth_bwd_body<LOGN, V>(U, abar, tw, *app, k, app->cout[k], blockIdx.x * Geo<LOGN, V>::RB, pgrad, K,
-                          sm_gbwd, red);
+    growth_bwd_body<LOGN, V>(U, abar, tw, *app, k, app->cout[k], blockIdx.x, stride, pgrad, K,
+                             sm_gbwd, red);
 }
 
 // ---------------------------------------------------------------------------
@@ -406,7 +439,7 @@ __global__ void __launch_bounds__(Geo<LOGN, V>::RT, 512 / Geo<LOGN, V>::RT) k_ro
     pdl_wait();
     pdl_launch_dependents();
     const int c = blockIdx.y, y0 = blockIdx.x * G::RB;
-    gather_rows<LOGN, V>(src + size_t(c) * G::M * G::N + y0, sm_c2ra);
+    gather_rows<G>(src + size_t(c) * G::M * G::N + y0, sm_c2ra);
     float* d = dst + (size_t(c) * G::N + y0) * G::N;
     auto out = [&](int s, int i, float2 v) {
         float2* p = reinterpret_cast<float2*>(d + size_t(s) * G::N) + i;
@@ -418,7 +451,7 @@ __global__ void __launch_bounds__(Geo<LOGN, V>::RT, 512 / Geo<LOGN, V>::RT) k_ro
         }
         *p = o;
     };
-    c2r_rows<LOGN, V>(sm_c2ra, tw, out);
+    c2r_rows<G>(sm_c2ra, tw, out);
 }
 
 // Plain inverse column FFT of a kx-major [planes][M][N] spectrum, in place.
@@ -448,7 +481,7 @@ cudaError_t prepare_backward_variant() {
                           reinterpret_cast<const void*>(k_col_conv_adj<LOGN, V>),
                           reinterpret_cast<const void*>(k_row_c2r_add<LOGN, V>),
                           reinterpret_cast<const void*>(k_col_inv<LOGN, V>)};
-    const size_t smem[5] = {DiffBwdGeo<LOGN, V>::SMEM, G::R2C_SMEM, AdjColGeo<LOGN, V>::SMEM,
+    const size_t smem[5] = {DiffBwdGeo<LOGN, V>::SMEM, GrowthRows<LOGN, V>::R2C_SMEM, AdjColGeo<LOGN, V>::SMEM,
                             G::R2C_SMEM, size_t(G::TW) * G::CP * sizeof(float2)};
     for (int i = 0; i < 5; ++i)
         if ((e = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -483,9 +516,9 @@ cudaError_t launch_diff_bwd(const BwdArgs& a, cudaStream_t st) {
 }
 template <int LOGN, int V>
 cudaError_t launch_growth_bwd(const BwdArgs& a, cudaStream_t st) {
-    using G = Geo<LOGN, V>;
+    using G = GrowthRows<LOGN, V>;
     return launch_pdl(k_growth_bwd<LOGN, V>, dim3(G::N / G::RB, a.K), G::RT, G::R2C_SMEM, st,
-                      a.U, a.abar, a.tw, a.ap, a.pgrad, a.K);
+                      a.U, a.abar, a.tw, a.ap, a.pgrad, a.K, a.var.chosen ? 8 : 32);
 }
 template <int LOGN, int V>
 cudaError_t launch_col_adj(const BwdArgs& a, cudaStream_t st) {
@@ -527,10 +560,10 @@ cudaError_t launch_backward(const BwdArgs& a, cudaStream_t st) {
     cudaError_t e = launch_diff_bwd<LOGN, kDiffBwdVariant>(a, st);
     if (e != cudaSuccess) return e;
     // the adjoint kernels exist in the CTA shapes of variants 0-2: the plan
-    // variants take the shape they share (row passes: two rows per CTA as
-    // in variant 2; column pass: Geo::CVS)
-    const int vrow = a.var.c2r > 2 ? 2 : a.var.c2r;
-    const int vcol = a.var.col == 3 ? 1 : (a.var.col == 4 ? 0 : a.var.col);
+    // variants take the shape they share (row passes: the fewest rows per
+    // CTA, as variant 0; column pass: Geo::CVS)
+    const int vrow = a.var.c2r > 2 ? 0 : a.var.c2r;
+    const int vcol = a.var.col > 2 ? a.var.col - 3 : a.var.col;
     CG_VARIANT_SWITCH(vrow, e = launch_growth_bwd, a, st)
     if (e != cudaSuccess) return e;
     CG_VARIANT_SWITCH(vcol, e = launch_col_adj, a, st)

@@ -53,7 +53,8 @@ int row_tile_rows(int v) {
         if (v == 3) return C2RShape<LOGN, 3>::RB;
         if (v == 4) return C2RShape<LOGN, 4>::RB;
     }
-    return v == 1 ? Geo<LOGN, 1>::RB : (v == 2 ? Geo<LOGN, 2>::RB : Geo<LOGN, 0>::RB);
+    return v == 1 ? C2RShape<LOGN, 1>::RB
+                  : (v == 2 ? C2RShape<LOGN, 2>::RB : C2RShape<LOGN, 0>::RB);
 }
 int row_tile_rows(int logn, int v) {
     switch (logn) {
@@ -115,17 +116,18 @@ __global__ void __launch_bounds__(Geo<LOGN, V>::CT, 512 / Geo<LOGN, V>::CT)
     kb_col_conv(const WorldDesc* __restrict__ worlds, const WorkItem* __restrict__ items, int count,
                 int* err) {
     extern __shared__ __align__(128) float2 smb_col[];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bar[Geo<LOGN, V>::NBUF];
     pdl_wait();
     pdl_launch_dependents();
-    init_tile_barrier(&bar);
+    init_tile_barriers<Geo<LOGN, V>::NBUF>(bar);
     uint32_t phase = 0;
     for (int i = blockIdx.x; i < count; i += gridDim.x) {
         __syncthreads();
         const WorkItem it = items[i];
         const WorldDesc& w = worlds[it.world];
         if (!col_conv_body<LOGN, V, KRE>(w.rowspec, w.kspec, w.kre, w.U, w.tw, w.groups, it.c,
-                                         it.a, smb_col, &bar, phase, err))
+                                         it.a, 0, w.groups.in_count[it.c], smb_col, bar, phase,
+                                         err, [] {}))
             return;   // a bounded wait timed out (uniform across the block)
     }
 }
@@ -135,17 +137,17 @@ __global__ void __launch_bounds__(C2RShape<LOGN, V>::RT, C2RShape<LOGN, V>::MINB
     kb_row_c2r_growth(const WorldDesc* __restrict__ worlds, const WorkItem* __restrict__ items,
                       int count, int* err) {
     extern __shared__ __align__(128) float2 smb_c2r[];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bar[C2RShape<LOGN, V>::NBUF];
     pdl_wait();
     pdl_launch_dependents();
-    init_tile_barrier(&bar);
+    init_tile_barriers<C2RShape<LOGN, V>::NBUF>(bar);
     uint32_t phase = 0;
     for (int i = blockIdx.x; i < count; i += gridDim.x) {
         __syncthreads();
         const WorkItem it = items[i];
         const WorldDesc& w = worlds[it.world];
         if (!row_c2r_growth_variant<LOGN, V>(&w.umap[V], true, w.A, w.tw, w.groups, w.gp,
-                                             w.temp, nullptr, 0.f, it.c, it.a, smb_c2r, &bar,
+                                             w.temp, nullptr, 0.f, it.c, it.a, smb_c2r, bar,
                                              phase, err))
             return;   // a bounded wait timed out (uniform across the block)
     }

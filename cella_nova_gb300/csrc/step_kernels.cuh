@@ -28,22 +28,22 @@
 namespace cg {
 
 // Geometry of one grid size.  V selects a variant (the autotuner times
-// them): row kernels V=1 / V=2 halve / quarter the rows per CTA and the
-// threads (the forward row pass's variant 2 streams variant 1's tile
-// instead, R2CShape); the column kernel V=1 halves and V=2 doubles the
-// columns and the threads per CTA (work per thread is unchanged); diffusion
-// V=1 keeps its sums in registers (DiffGeoReg, 16-row strips; V=3 the same
-// in 8-row strips, DiffTile) and V=2 uses 64 tile rows with two columns per
-// thread instead of 32 rows (the diffusion adjoint takes V=1 as 16 tile
-// rows).  Variants 0-2, and diffusion's 3, compute the same bits.
+// them; 0 is what a world runs untuned, so it is the shape that measured
+// best): the inverse row pass takes the fewest rows and threads per CTA with
+// V=0, twice and four times as many with V=1 and V=2; the forward row pass
+// the other way round (R2CShape; its variant 2 streams variant 1's tile
+// from side 1024 on); the column kernel takes the fewest columns and threads
+// per CTA with V=0, twice as many with V=1, four times with V=2 (work per
+// thread is unchanged).  Diffusion's variants are DiffTile's.  Variants 0-2,
+// and diffusion's 3, compute the same bits.
 //
 // Variants 3 and 4 (grid sides of at least kMinPairLogN) change the FFT
 // plans instead of only the shapes, and agree with the others to rounding:
 // the row passes transform two real rows as one complex sequence of length
 // n (PairGeo, pair_rows.cuh) with radix-16 (V=3) or radix-8 (V=4) plans;
 // the column pass runs the remainder-first plan forward and the greedy plan
-// inverse (the order of variants 0-2 reversed) in the CTA shape of V=1
-// (V=3) or V=0 (V=4).  Layouts in memory do not depend on V.
+// inverse (the order of variants 0-2 reversed) in the CTA shape of V=0
+// (V=3) or V=1 (V=4).  Layouts in memory do not depend on V.
 template <int LOGN, int V = 0>
 struct Geo {
     static_assert(V >= 0 && V <= 4, "variant");
@@ -56,10 +56,22 @@ struct Geo {
     // pass) conflict-free: odd for RB >= 16 (16 rows of one column), 2 mod 16
     // for RB = 8 (8 rows x 2 columns), 4 mod 16 for RB = 4, 8 mod 16 for
     // RB = 2 (2 rows x 8 columns).
-    static constexpr int RB0 = 8192 / M;
-    static constexpr int RB1 = RB0 < 8 ? 8 : (RB0 > N ? N : RB0);
-    static constexpr int RB = (V == 1) ? RB1 / 2 : (V == 2 ? RB1 / 4 : RB1);
-    static constexpr int RT = (V == 0) ? 512 : (V == 1 ? 256 : 128);
+    //
+    // From side 1024 on the CTAs of 128 threads (V=0) won the inverse row
+    // pass: 57.5 against 65.7 and 87.1 us at 2048^2 with C=3, K=9, and 17.0
+    // against 19.2 and 31.1 us at 1024^2.  Up to side 512 a whole world is
+    // less work than the GPU has places for, so what counts is the number of
+    // CTAs and the length of each one's chain: 4, 8 or 16 rows per CTA, a
+    // thread per radix-16 butterfly, and at least a warp (at 256^2 4.6 us
+    // with 4 rows and 5.5 us with 16; 64 rows and 512 threads, which fill a
+    // channel with 4 CTAs, took 14.0 us).
+    static constexpr bool SMALL = LOGN <= kMaxSmallLogN;
+    static constexpr int TPR = M < 16 ? 1 : M / 16;   // threads per row
+    static constexpr int RBS = (V == 1) ? 8 : (V == 2 ? 16 : 4);
+    static constexpr int RB0 = 8192 / M < 8 ? 8 : 8192 / M;
+    static constexpr int RB = SMALL ? RBS : (V == 1) ? RB0 / 2 : (V == 2 ? RB0 : RB0 / 4);
+    static constexpr int RT = SMALL ? (RBS * TPR < 32 ? 32 : RBS * TPR)
+                                    : (V == 1) ? 256 : (V == 2 ? 512 : 128);
     static constexpr int ROW_MR = 16;
     static constexpr int RP = padded_len(M) + (RB >= 16 ? 1 : (RB == 8 ? 2 : (RB == 4 ? 4 : 8)));
     static constexpr size_t R2C_SMEM = size_t(RB) * RP * sizeof(float2);
@@ -71,34 +83,40 @@ struct Geo {
     static constexpr int C2R_TILE = RB * M;
     static_assert((C2R_TILE * sizeof(float2)) % 128 == 0 && (RB * UBOX * sizeof(float2)) % 128 == 0,
                   "tensor-copy destination alignment");
-    static constexpr size_t C2R_SMEM = (size_t(C2R_LAND) + size_t(C2R_TILE)) * sizeof(float2);
+    // Small sides keep two tiles in flight (the next kernel's lands during the
+    // current one's transform); at larger ones the second tile costs resident
+    // CTAs, and the step was 10-15 us slower with it at 2048^2.
+    static constexpr int NBUF = SMALL ? 2 : 1;
+    static constexpr size_t C2R_SMEM =
+        (size_t(C2R_LAND) + size_t(NBUF) * C2R_TILE) * sizeof(float2);
     static_assert(C2R_SMEM <= 227 * 1024, "inverse row pass shared memory");
-    // Column kernel: TW columns per CTA, CT threads; a padded work buffer
-    // and an unpadded staging tile that bulk copies fill.  TW = 4096/N keeps
-    // 256 butterflies per radix-16 pass (one per thread) at every size.
-    // CVS: the CTA shape of the column pass (V=3 takes V=1's, V=4 V=0's);
+    // Column kernel: TW columns per CTA, CT threads (one per butterfly of a
+    // radix-16 pass); a padded work buffer and an unpadded staging tile that
+    // bulk copies fill.  From side 1024 on TW = 2048/N and 128 threads with
+    // V=0 (2048^2: 56.7 against 68.4 and 84.3 us; 1024^2: 17.0 against 19.5
+    // and 26.9 us); up to side 512 4, 2 or 8 columns (256^2: 2.9 us, and
+    // 7.8 us with 16 columns and 256 threads).
+    // CVS: the CTA shape of the column pass (V=3 takes V=0's, V=4 V=1's);
     // COL_SWAP: the remainder-first plan forward, the greedy plan inverse.
-    static constexpr int CVS = (V == 3) ? 1 : (V == 4 ? 0 : V);
+    static constexpr int CVS = (V >= 3) ? V - 3 : V;
     static constexpr bool COL_SWAP = (V >= 3);
-    static constexpr int TW0 = 4096 / N;
-    static constexpr int TW1 = TW0 < 2 ? 2 : (TW0 > M ? M : TW0);
-    static constexpr int TW = (CVS == 1) ? (TW1 > 1 ? TW1 / 2 : 1)
-                                         : (CVS == 2 ? (2 * TW1 > M ? M : 2 * TW1) : TW1);
-    static constexpr int CT = (CVS == 1) ? 128 : (CVS == 2 ? 512 : 256);
+    static constexpr int TWS = (CVS == 1) ? 2 : (CVS == 2 ? 8 : 4);
+    static constexpr int TW = SMALL ? TWS : (2048 / N) << CVS;
+    static constexpr int CT = SMALL ? (TWS * N / 16 < 32 ? 32 : TWS * N / 16) : 128 << CVS;
     // Resident CTAs per SM the compiler must allow for (the register cap) in
-    // the single-world column pass: the small-CTA variant asks for five, which
+    // the single-world column pass: variants 0 and 3 ask for five, which
     // ptxas meets without spills (96 registers at n = 2048; 66.0 against
     // 67.6 us).  Six CTAs of the swapped-plan variant 3 (80 registers, no
     // spills) ran at 62.1 against 61.1 us, so it keeps five.  On the inverse
     // row pass, three CTAs of 256 threads (80 registers) ran at 121 against
     // 92 us and five of the 128-thread variant at 63.5 against 63.7 us; only
     // the paired variant 3 takes a cap there (pair_rows.cuh).
-    static constexpr int COL_MINB = (CVS == 1) ? 5 : 512 / CT;
+    static constexpr int COL_MINB = (CVS == 0 && !SMALL) ? 5 : 512 / CT;
     static constexpr int CP = padded_len(N) + 1;
     // the staging tile is a bulk-copy (TMA) destination: 16-byte aligned
     static constexpr int KSOFF = (TW * CP + 1) & ~1;
     static_assert((KSOFF * sizeof(float2)) % 16 == 0, "bulk-copy destination alignment");
-    static constexpr size_t COL_SMEM = (size_t(KSOFF) + size_t(TW) * N) * sizeof(float2);
+    static constexpr size_t COL_SMEM = (size_t(KSOFF) + size_t(NBUF) * TW * N) * sizeof(float2);
     // Twiddle buffer: W_N^m (m < N), then the pass tables of the column
     // forward plan (greedy radix 16, length N), the column inverse plan
     // (remainder first), the row plan (greedy, length M) and the radix-8
@@ -110,7 +128,7 @@ struct Geo {
     static constexpr int TW_TOTAL = TW_PAIR8 + tw_size(N, false, 8);
     // Diffusion tile.
     static constexpr int TX = N < 64 ? N : 64;
-    static constexpr int TY0 = (V == 1) ? 16 : (V == 2 ? 64 : 32);
+    static constexpr int TY0 = (V == 2) ? (SMALL ? 32 : 64) : 16;
     static constexpr int TY = N < TY0 ? N : TY0;
 };
 
@@ -131,9 +149,8 @@ namespace cg {
 // t / RB + i * (RT / RB), so both the padded shared index pidx(kx) and the
 // global address advance by constants (pidx(kx + STEP) = pidx(kx) +
 // pidx(STEP) when STEP is a multiple of 16).  f(s, kx, pidx(kx)).
-template <int LOGN, int V, class F>
+template <class G, class F>
 __device__ __forceinline__ void for_row_tile(F f) {
-    using G = Geo<LOGN, V>;
     static_assert(G::RT % G::RB == 0, "a thread keeps one row");
     constexpr int STEP = G::RT / G::RB;
     const int s = threadIdx.x % G::RB, kx0 = threadIdx.x / G::RB;
@@ -146,9 +163,13 @@ __device__ __forceinline__ void for_row_tile(F f) {
     }
 }
 
-template <int LOGN, int V = 0>
+// Row s of a CTA's rows, counted from its first.
+struct RowsInOrder {
+    __device__ __forceinline__ int operator()(int s) const { return s; }
+};
+template <class G, class ROW = RowsInOrder>
 __device__ __forceinline__ void r2c_finish(float2* sm, const float2* __restrict__ tw,
-                                           float2* __restrict__ dst);
+                                           float2* __restrict__ dst, ROW row = ROW());
 
 template <int LOGN, int V = 0>
 __device__ __forceinline__ void row_r2c_body(const float* __restrict__ state,
@@ -163,22 +184,21 @@ __device__ __forceinline__ void row_r2c_body(const float* __restrict__ state,
     // the first pass reads global memory: no load-store barrier
     FftPasses<G::M, 1, false, G::RT, G::RB, false, G::ROW_MR, false, false, true>::run(
         ld0, rows, rows, rows, tw + G::TW_ROW);
-    r2c_finish<LOGN, V>(sm, tw, rowspec + size_t(c) * G::M * G::N + y0);
+    r2c_finish<G>(sm, tw, rowspec + size_t(c) * G::M * G::N + y0);
 }
 
 // Even/odd split of RB transformed rows in shared memory (X[k] from Z[k],
 // Z[M-k]; X[0], X[M] packed in slot 0), stored straight to the kx-major
-// rows dst[kx * N + s].  The row index runs fastest over the threads, so RB
+// rows dst[kx * N + row(s)].  The row index runs fastest over the threads, so RB
 // consecutive lanes write one column's RB rows (a full sector for RB = 4),
 // and the shared reads stay conflict-free with the row pitch RP.
-template <int LOGN, int V>
+template <class G, class ROW>
 __device__ __forceinline__ void r2c_finish(float2* sm, const float2* __restrict__ tw,
-                                           float2* __restrict__ dst) {
-    using G = Geo<LOGN, V>;
+                                           float2* __restrict__ dst, ROW row) {
     constexpr int H = G::M / 2, RB = G::RB;
     auto split = [&](int s, int k, float2& lo, float2& hi) {   // X[k], conj X[M-k] for 0 < k <= H
-        const float2* row = sm + s * G::RP;
-        const float2 a = row[pidx(k)], b = row[pidx(G::M - k)];
+        const float2* z = sm + s * G::RP;
+        const float2 a = z[pidx(k)], b = z[pidx(G::M - k)];
         const float2 E = make_float2(a.x + b.x, a.y - b.y);
         const float2 D = make_float2(a.x - b.x, a.y + b.y);
         const float2 O = make_float2(D.y, -D.x);
@@ -191,19 +211,19 @@ __device__ __forceinline__ void r2c_finish(float2* sm, const float2* __restrict_
     if (threadIdx.x < RB) {
         const int s = threadIdx.x;
         const float2 z = sm[s * G::RP];
-        dst[s] = make_float2(2.f * (z.x + z.y), 2.f * (z.x - z.y));
+        dst[row(s)] = make_float2(2.f * (z.x + z.y), 2.f * (z.x - z.y));
     } else if (threadIdx.x < 2 * RB) {
         const int s = threadIdx.x - RB;
         float2 lo, hi;
         split(s, H, lo, hi);
-        dst[size_t(H) * G::N + s] = lo;
+        dst[size_t(H) * G::N + row(s)] = lo;
     }
     for (int item = threadIdx.x + RB; item < RB * H; item += G::RT) {
         const int s = item % RB, k = item / RB;
         float2 lo, hi;
         split(s, k, lo, hi);
-        dst[size_t(k) * G::N + s] = lo;
-        dst[size_t(G::M - k) * G::N + s] = hi;
+        dst[size_t(k) * G::N + row(s)] = lo;
+        dst[size_t(G::M - k) * G::N + row(s)] = hi;
     }
 }
 
@@ -216,7 +236,7 @@ __device__ __forceinline__ void row_r2c_variant(const float* __restrict__ state,
     if constexpr (R2CShape<LOGN, V>::PAIR)
         pair_r2c_body<typename R2CShape<LOGN, V>::P>(state, rowspec, tw, c, y0, sm);
     else
-        row_r2c_body<LOGN, V>(state, rowspec, tw, c, y0, sm);
+        row_r2c_body<LOGN, R2CShape<LOGN, V>::GV>(state, rowspec, tw, c, y0, sm);
 }
 
 __device__ __forceinline__ void init_tile_barrier(uint64_t* bar) {
@@ -225,6 +245,28 @@ __device__ __forceinline__ void init_tile_barrier(uint64_t* bar) {
         fence_barrier_init();
     }
     __syncthreads();
+}
+
+template <int NB>
+__device__ __forceinline__ void init_tile_barriers(uint64_t* bar) {
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 0; i < NB; ++i) mbar_init(bar + i, 1);
+        fence_barrier_init();
+    }
+    __syncthreads();
+}
+
+// Bring `count` float2 of a twiddle table into this SM's L1: on a small side
+// a pass would otherwise wait for its first look at them in L2 (about as
+// long as the pass itself), and a kernel can do it before it waits for the
+// kernel it depends on.
+template <int T>
+__device__ __forceinline__ void warm_table(const float2* __restrict__ t, int count) {
+    for (int i = threadIdx.x * 16; i < count; i += T * 16) {   // a 128-byte line each
+        float v;
+        asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(t + i));
+    }
 }
 
 // The streaming form of the forward row pass (R2CShape<LOGN, 2>): this CTA
@@ -277,7 +319,7 @@ __device__ __forceinline__ bool row_r2c_stream(ITEM item, int count,
             ld0, rows, rows, rows, tw + G::TW_ROW, [&]() {
                 if (i + int(gridDim.x) < count) issue(i + gridDim.x);
             });
-        r2c_finish<LOGN, 1>(sm, tw, dst);
+        r2c_finish<G>(sm, tw, dst);
         __syncthreads();
     }
     return true;
@@ -292,6 +334,10 @@ __global__ void __launch_bounds__(R2CShape<LOGN, V>::RT, R2CShape<LOGN, V>::MINB
               const float2* __restrict__ tw, int cbase, int nc, int* err) {
     extern __shared__ __align__(128) float2 sm_r2c[];
     using Sh = R2CShape<LOGN, V>;
+    if constexpr (LOGN <= kMaxSmallLogN && !Sh::PAIR) {
+        warm_table<Sh::RT>(tw + Geo<LOGN>::TW_ROW, tw_size(1 << (LOGN - 1), false));
+        warm_table<Sh::RT>(tw, 1 << (LOGN - 2));   // W_N^k of the split
+    }
     pdl_wait();
     pdl_launch_dependents();
     if constexpr (Sh::STREAM) {
@@ -330,7 +376,7 @@ __global__ void __launch_bounds__(R2CShape<LOGN, V>::RT, R2CShape<LOGN, V>::MINB
 //   P(ky) alpha(ky) + conj P(-ky) beta(ky),
 // alpha/beta = (K(.,0) +- K(.,n/2))/2 (prepared by k_pack_kernel); P(-ky)
 // lives in another thread, so that tile swaps column 0 through W first.
-// grid (M/TW, C), block CT.
+// grid (M/TW, C, Z), block CT: at small sides Z CTAs share a tile's kernels.
 // ---------------------------------------------------------------------------
 // Returns false if a bounded wait timed out (the error word is set).  `bar`
 // is an initialised mbarrier owned by the caller and `phase` counts its
@@ -338,54 +384,72 @@ __global__ void __launch_bounds__(R2CShape<LOGN, V>::RT, R2CShape<LOGN, V>::MINB
 // KRE: the kernel spectra are real (point-symmetric kernels) and come from
 // kre, the real parts of kspec: half the bytes per kernel tile, and each
 // product is two multiplications instead of a complex one.
-template <int LOGN, int V = 0, bool KRE = false>
+// The tiles of a column pass are stages 0 (the input columns) and 1 + gi
+// (kernel gi of [g0, g1) of the channel's kernels); stage q of the CTA's life
+// (`phase` counts them) uses staging buffer q % NBUF and its mbarrier, and is
+// issued as soon as stage q - NBUF has been read.  start() runs between the
+// issue of the first kernel's tile (NBUF = 2) and that of the input columns:
+// the spectra do not depend on the kernels before this one in the stream (what
+// wrote them completed before the forward row pass began), so their copy
+// overlaps the wait for the row spectra.
+template <int LOGN, int V = 0, bool KRE = false, class START>
 __device__ __forceinline__ bool col_conv_body(const float2* __restrict__ rowspec,
                                               const float2* __restrict__ kspec,
                                               const float* __restrict__ kre,
                                               float2* __restrict__ U,
                                               const float2* __restrict__ tw,
-                                              const KernelGroups& groups, int c, int kx0,
-                                              float2* sm, uint64_t* barp, uint32_t& phase,
-                                              int* err) {
+                                              const KernelGroups& groups, int c, int kx0, int g0,
+                                              int g1, float2* sm, uint64_t* barp, uint32_t& phase,
+                                              int* err, START start) {
     using G = Geo<LOGN, V>;
-    constexpr int N = G::N, M = G::M, TW = G::TW, T = G::CT;
-    const int cnt = groups.in_count[c];
-    if (cnt == 0) return true;
+    constexpr int N = G::N, M = G::M, TW = G::TW, T = G::CT, NBUF = G::NBUF;
+    const int base = groups.in_start[c] + g0, cnt = g1 - g0;
     float2* W = sm;
     float2* KS = sm + G::KSOFF;
-    const float* KR = reinterpret_cast<const float*>(KS);   // the real kernel tile (KRE)
-    uint64_t& bar = *barp;
-    const int base = groups.in_start[c];
     constexpr uint32_t kTileBytes = uint32_t(TW) * N * sizeof(float2);
     constexpr uint32_t kKernelBytes = KRE ? uint32_t(TW) * N * sizeof(float) : kTileBytes;
-    auto issue_bytes = [&](const void* src, uint32_t bytes) {   // all threads call; thread 0 copies
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            mbar_arrive_expect_tx(&bar, bytes);
-            bulk_g2s(KS, src, bytes, &bar);
+    const uint32_t q0 = phase;
+    auto buffer = [&](uint32_t q) { return KS + (NBUF == 2 ? (q & 1u) * (TW * N) : 0); };
+    auto issue = [&](int stage) {   // thread 0 copies, after a barrier that closed the buffer's reads
+        if (threadIdx.x != 0) return;
+        uint64_t* bar = barp + (NBUF == 2 ? (q0 + stage) & 1u : 0);
+        float2* dst = buffer(q0 + stage);
+        if (stage == 0) {
+            mbar_arrive_expect_tx(bar, kTileBytes);
+            bulk_g2s(dst, rowspec + (size_t(c) * M + kx0) * N, kTileBytes, bar);
+        } else {
+            const size_t off = (size_t(groups.in_idx[base + stage - 1]) * (M + 1) + kx0) * N;
+            mbar_arrive_expect_tx(bar, kKernelBytes);
+            if constexpr (KRE) bulk_g2s(dst, kre + off, kKernelBytes, bar);
+            else bulk_g2s(dst, kspec + off, kKernelBytes, bar);
         }
     };
-    auto issue = [&](const float2* src) { issue_bytes(src, kTileBytes); };
+    auto issue_next = [&](int stage) {   // all threads call, after reading stage - NBUF
+        fence_proxy_async_smem();
+        __syncthreads();
+        if (stage <= cnt) issue(stage);
+    };
     auto wait_tile = [&]() -> bool {
-        const bool ok = mbar_wait(&bar, phase & 1, err);
+        uint64_t* bar = barp + (NBUF == 2 ? phase & 1u : 0);
+        const uint32_t parity = (NBUF == 2 ? phase >> 1 : phase) & 1u;
+        const bool ok = mbar_wait(bar, parity, err);
         if (__syncthreads_or(!ok)) {
-            // give the copy in flight one more bounded chance to land before
+            // give the copies in flight one more bounded chance to land before
             // this CTA's shared memory is released
-            mbar_wait(&bar, phase & 1, nullptr);
+            mbar_wait(bar, parity, nullptr);
+            if (NBUF == 2 && int(phase - q0) < cnt)
+                mbar_wait(barp + ((phase + 1) & 1u), ((phase + 1) >> 1) & 1u, nullptr);
             return false;
         }
         ++phase;
         return true;
     };
-    auto issue_kernel = [&](int gi) {
-        const int k = groups.in_idx[base + gi];
-        const size_t off = (size_t(k) * (M + 1) + kx0) * N;
-        if constexpr (KRE) issue_bytes(kre + off, kKernelBytes);
-        else issue_bytes(kspec + off, kKernelBytes);
-    };
 
-    issue(rowspec + (size_t(c) * M + kx0) * N);
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (NBUF == 2 && cnt > 0) issue(1);
+    start();
+    issue(0);
     if (!wait_tile()) return false;
 
     // forward plan: greedy (variants 0-2) or remainder first (COL_SWAP);
@@ -399,16 +463,19 @@ __device__ __forceinline__ bool col_conv_body(const float2* __restrict__ rowspec
     constexpr int JL = N / RL;
     constexpr int IPTL = (TW * JL + T - 1) / T;
     float2 F[IPTL][RL];
-    auto ld_in = [&](int s, int i, int, int) { return KS[s * N + i]; };
+    const float2* in = buffer(q0);
+    auto ld_in = [&](int s, int i, int, int) { return in[s * N + i]; };
     SmemRows wrows{W, G::CP};
     auto keep = [&](int, int, float2 v, int it, int r) { F[it][r] = v; };
     // forward: the first pass reads the staging tile, the last one keeps its
     // values in registers (no load-store barriers)
     fft_with_hook<N, false, T, TW, FREM, 16, false, false, false>(
-        ld_in, wrows, wrows, keep, tw_fwd, [&]() { issue_kernel(0); });
+        ld_in, wrows, wrows, keep, tw_fwd, [&]() { issue_next(NBUF); });
 
     for (int gi = 0; gi < cnt; ++gi) {
         if (!wait_tile()) return false;
+        const float2* KT = buffer(phase - 1);   // this kernel's tile
+        const float* KR = reinterpret_cast<const float*>(KT);   // ... of real values (KRE)
         if (kx0 == 0) {   // publish column 0 for the conj P(-ky) reads
 #pragma unroll
             for (int it = 0; it < IPTL; ++it) {
@@ -449,7 +516,7 @@ __device__ __forceinline__ bool col_conv_body(const float2* __restrict__ rowspec
                     }
                     return make_float2(__fmul_rn(p.x, kv), __fmul_rn(p.y, kv));
                 } else {
-                    const float2 kv = KS[s * N + i];
+                    const float2 kv = KT[s * N + i];
                     if (C0 && s == 0) {
                         const float2 pm = cconj(W[pidx((N - i) & (N - 1))]);
                         return cadd(cmul(p, kv), cmul(pm, __ldg(&kb[i])));
@@ -459,7 +526,7 @@ __device__ __forceinline__ bool col_conv_body(const float2* __restrict__ rowspec
             };
             fft_with_hook<N, true, T, TW, !FREM, 16, false, C0, false>(
                 ld_mul, wrows, wrows, gst, tw_inv, [&]() {
-                if (gi + 1 < cnt) issue_kernel(gi + 1);
+                if (gi + NBUF < cnt) issue_next(gi + 1 + NBUF);
             });
         };
         if (kx0 == 0)
@@ -477,15 +544,30 @@ __global__ void __launch_bounds__(Geo<LOGN, V>::CT, Geo<LOGN, V>::COL_MINB)
                const float2* __restrict__ tw, const __grid_constant__ KernelGroups groups,
                int* err, int cbase) {
     extern __shared__ __align__(128) float2 sm_col[];
-    __shared__ __align__(8) uint64_t bar;
-    pdl_wait();
-    pdl_launch_dependents();
+    using G = Geo<LOGN, V>;
+    __shared__ __align__(8) uint64_t bar[G::NBUF];
     const int c = blockIdx.y + cbase;
-    if (groups.in_count[c] == 0) return;
-    init_tile_barrier(&bar);
+    const int n = groups.in_count[c];
+    // gridDim.z CTAs share a tile's kernels (launch_col)
+    const int g0 = n * int(blockIdx.z) / int(gridDim.z);
+    const int g1 = n * int(blockIdx.z + 1) / int(gridDim.z);
+    if constexpr (!G::SMALL) pdl_wait();
+    if constexpr (!G::SMALL) pdl_launch_dependents();
+    if (g0 == g1) {
+        if constexpr (G::SMALL) pdl_wait();
+        return;
+    }
+    init_tile_barriers<G::NBUF>(bar);
+    if constexpr (G::SMALL)
+        warm_table<G::CT>(tw + G::TW_COL_FWD, tw_size(G::N, false) + tw_size(G::N, true));
     uint32_t phase = 0;
-    col_conv_body<LOGN, V, KRE>(rowspec, kspec, kre, U, tw, groups, c,
-                                blockIdx.x * Geo<LOGN, V>::TW, sm_col, &bar, phase, err);
+    col_conv_body<LOGN, V, KRE>(rowspec, kspec, kre, U, tw, groups, c, blockIdx.x * G::TW, g0, g1,
+                                sm_col, bar, phase, err, [&]() {
+                                    if constexpr (G::SMALL) {
+                                        pdl_wait();
+                                        pdl_launch_dependents();
+                                    }
+                                });
 }
 
 // ---------------------------------------------------------------------------
@@ -525,7 +607,7 @@ __device__ __forceinline__ bool row_c2r_growth_body(const CUtensorMap* umap, boo
                                                     int c, int y0, float2* sm, uint64_t* barp,
                                                     uint32_t& phase, int* err) {
     using G = Geo<LOGN, V>;
-    constexpr int M = G::M, RB = G::RB;
+    constexpr int M = G::M, RB = G::RB, NBUF = G::NBUF;
     constexpr int RL = last_radix(M, G::ROW_MR);
     constexpr int JL = M / RL;
     constexpr int ITEMS = RB * JL;
@@ -534,26 +616,32 @@ __device__ __forceinline__ bool row_c2r_growth_body(const CUtensorMap* umap, boo
     static_assert(G::RT % RB == 0, "a thread keeps one row in every pass");
     const int cnt = groups.out_count[c], base = groups.out_start[c];
     float2* land = sm + G::C2R_LAND;
-    uint64_t& bar = *barp;
     if (umap_global && threadIdx.x == 0) tensormap_acquire(umap);
 
-    auto issue = [&](int gi) {   // all threads call; thread 0 copies
+    // the tile of kernel gi is stage q0 + gi of the CTA's life: landing tile
+    // and mbarrier (q0 + gi) % NBUF, issued once stage q0 + gi - NBUF was read
+    const uint32_t q0 = phase;
+    auto tile = [&](uint32_t q) { return land + (NBUF == 2 ? (q & 1u) * G::C2R_TILE : 0); };
+    auto issue = [&](int gi) {   // thread 0 copies
+        if (threadIdx.x != 0) return;
         const int k = groups.out_idx[base + gi];
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            mbar_arrive_expect_tx(&bar, kTileBytes);
+        uint64_t* bar = barp + (NBUF == 2 ? (q0 + gi) & 1u : 0);
+        float2* dst = tile(q0 + gi);
+        mbar_arrive_expect_tx(bar, kTileBytes);
 #pragma unroll
-            for (int q = 0; q < M / G::UBOX; ++q)
-                tensor2d_g2s(land + q * G::UBOX * RB, umap, 2 * y0, k * M + q * G::UBOX, &bar);
-        }
+        for (int q = 0; q < M / G::UBOX; ++q)
+            tensor2d_g2s(dst + q * G::UBOX * RB, umap, 2 * y0, k * M + q * G::UBOX, bar);
     };
-    auto wait_tile = [&]() -> bool {
-        const bool ok = mbar_wait(&bar, phase & 1u, err);
+    auto wait_tile = [&](int gi) -> bool {
+        uint64_t* bar = barp + (NBUF == 2 ? phase & 1u : 0);
+        const uint32_t parity = (NBUF == 2 ? phase >> 1 : phase) & 1u;
+        const bool ok = mbar_wait(bar, parity, err);
         if (__syncthreads_or(!ok)) {
-            // give the copy in flight one more bounded chance to land before
+            // give the copies in flight one more bounded chance to land before
             // this CTA's shared memory is released
-            mbar_wait(&bar, phase & 1u, nullptr);
+            mbar_wait(bar, parity, nullptr);
+            if (NBUF == 2 && gi + 1 < cnt)
+                mbar_wait(barp + ((phase + 1) & 1u), ((phase + 1) >> 1) & 1u, nullptr);
             return false;
         }
         ++phase;
@@ -569,10 +657,14 @@ __device__ __forceinline__ bool row_c2r_growth_body(const CUtensorMap* umap, boo
     // this thread's row: the same in every pass (RT is a multiple of RB)
     const int srow = threadIdx.x % RB;
     SmemRows rows{sm, G::RP};
-    if (cnt > 0) issue(0);
+    fence_proxy_async_smem();
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NBUF; ++i)
+        if (i < cnt) issue(i);
     for (int gi = 0; gi < cnt; ++gi) {
-        if (!wait_tile()) return false;
-        const float2* lt = land + srow;   // lt[kx * RB]
+        if (!wait_tile(gi)) return false;
+        const float2* lt = tile(phase - 1) + srow;   // lt[kx * RB]
         // m = j + q (M / R): m = 0 only in slot q = 0 (compile-time)
         auto ld0 = [&](int, int m, int, int q) -> float2 {
             if (q == 0 && m == 0) {
@@ -602,7 +694,11 @@ __device__ __forceinline__ bool row_c2r_growth_body(const CUtensorMap* umap, boo
         // values in registers: neither needs its load-store barrier
         fft_with_hook<M, true, G::RT, RB, false, G::ROW_MR, true, false, false>(
             ld0, rows, rows, gst, tw + G::TW_ROW, [&]() {
-                if (gi + 1 < cnt) issue(gi + 1);   // the first pass has read the tile
+                if (gi + NBUF < cnt) {   // the first pass has read the tile
+                    fence_proxy_async_smem();
+                    __syncthreads();
+                    issue(gi + NBUF);
+                }
             });
     }
 
@@ -653,14 +749,19 @@ __global__ void __launch_bounds__(C2RShape<LOGN, V>::RT, C2RShape<LOGN, V>::MINB
                      const GrowthParams* __restrict__ gp, float temp, float* __restrict__ udbg,
                      float udbg_scale, int* err, int cbase) {
     extern __shared__ __align__(128) float2 sm_c2r[];
-    __shared__ __align__(8) uint64_t bar;
+    using Sh = C2RShape<LOGN, V>;
+    __shared__ __align__(8) uint64_t bar[Sh::NBUF];
+    init_tile_barriers<Sh::NBUF>(bar);
+    if constexpr (LOGN <= kMaxSmallLogN && !Sh::PAIR) {
+        warm_table<Sh::RT>(tw + Geo<LOGN>::TW_ROW, tw_size(1 << (LOGN - 1), false));
+        warm_table<Sh::RT>(tw, 1 << (LOGN - 1));   // W_N^m of the pre-split
+    }
     pdl_wait();
     pdl_launch_dependents();
-    init_tile_barrier(&bar);
     uint32_t phase = 0;
     row_c2r_growth_variant<LOGN, V, DBG>(&umap, false, A, tw, groups, *gp, temp, udbg, udbg_scale,
-                                    blockIdx.y + cbase, blockIdx.x * C2RShape<LOGN, V>::RB,
-                                    sm_c2r, &bar, phase, err);
+                                    blockIdx.y + cbase, blockIdx.x * Sh::RB, sm_c2r, bar, phase,
+                                    err);
 }
 
 // ---------------------------------------------------------------------------
@@ -1062,16 +1163,23 @@ __device__ __forceinline__ void diffusion_reg_body(const float* __restrict__ A,
     }
 }
 
-// The diffusion phase's variants: 0 the shared-memory tile body, 1 and 3
-// the register body in 16- and 8-row strips, 2 the column-pair body.  All
-// four give the same bits.  TX x TY is the tile of one CTA (one work item).
+// The diffusion phase's variants: 1 and 3 the register body in 16- and 8-row
+// strips, 2 the column-pair body, 0 the shared-memory tile body up to side
+// 512 (at 256^2 2.5 us, against 7.0 and 4.1 us for the strips, whose rows
+// wait for their loads one after another) and the register body from 1024
+// on: there launch_diff takes 16-row strips where their CTAs fill the GPU at
+// least once and 8-row strips otherwise (2048^2: 35.0 against 39.2 us with
+// three channels, 15.6 against 10.6 us with one; 1024^2, C=3: 9.5 against
+// 9.1 us).  All give the same bits.  TX x TY is the tile of one CTA (one
+// work item).
 constexpr int kDiffVariants = 4;
-template <int LOGN, int V, int KIND = (V == 1 || V == 3) ? 1 : (V == 2 ? 2 : 0)>
+template <int LOGN, int V,
+          int KIND = V == 2 ? 2 : (V == 1 || V == 3 || LOGN > kMaxSmallLogN) ? 1 : 0>
 struct DiffTile;
 template <int LOGN, int V>
 struct DiffTile<LOGN, V, 1> {
     static constexpr bool REG = true, PAIR = false;
-    static constexpr int STRIP = (V == 3) ? 8 : 16;
+    static constexpr int STRIP = (V == 3 || (V == 0 && LOGN == 10)) ? 8 : 16;
     using D = DiffGeoReg<LOGN, STRIP>;
     static constexpr int THREADS = D::THREADS, TX = D::TX, TY = D::TY;
     static constexpr size_t SMEM = 0;
@@ -1235,10 +1343,21 @@ cudaError_t launch_r2c(const StepArgs& a, int c_lo, int nc, cudaStream_t st) {
     return launch_pdl(k_row_r2c<LOGN, V>, grid, R::RT, R::SMEM, st, a.x_in, a.rowspec, a.tw, c_lo,
                       nc, a.err);
 }
+// CTAs of the column pass that a small world's launch may fill the GPU with.
+constexpr int kSmallPlaces = 152 * 4;
 template <int LOGN, int V>
 cudaError_t launch_col(const StepArgs& a, int c_lo, int nc, cudaStream_t st) {
     using G = Geo<LOGN, V>;
-    const dim3 grid(G::M / G::TW, nc);
+    dim3 grid(G::M / G::TW, nc);
+    if constexpr (G::SMALL) {
+        // a tile's kernels spread over gridDim.z CTAs (each transforms the
+        // tile's input columns again) while all channels' CTAs leave places
+        int most = 1;
+        for (int c = c_lo; c < c_lo + nc; ++c)
+            most = a.groups.in_count[c] > most ? a.groups.in_count[c] : most;
+        const int places = kSmallPlaces / (G::M / G::TW * a.C);
+        grid.z = places < 1 ? 1 : (places < most ? places : most);
+    }
     if (a.kre)
         return launch_pdl(k_col_conv<LOGN, V, true>, grid, G::CT, G::COL_SMEM, st, a.rowspec,
                           a.kspec, a.kre, a.U, a.tw, a.groups, a.err, c_lo);
@@ -1267,6 +1386,12 @@ template <int LOGN, int V>
 cudaError_t launch_diff(const StepArgs& a, int c_lo, int nc, cudaStream_t st) {
     constexpr int N = 1 << LOGN;
     using D = DiffTile<LOGN, V>;
+    if constexpr (V == 0 && D::REG) {
+        // all channels' CTAs of 16-row strips (six fit an SM's registers)
+        constexpr int kTiles = N / DiffTile<LOGN, 1>::TX * (N / DiffTile<LOGN, 1>::TY);
+        if (kTiles * a.C < 6 * 152) return launch_diff<LOGN, 3>(a, c_lo, nc, st);
+        return launch_diff<LOGN, 1>(a, c_lo, nc, st);
+    }
     return launch_pdl(k_diffusion<LOGN, V>, dim3(N / D::TX, N / D::TY, nc), D::THREADS,
                       D::SMEM, st, a.A, a.x_in, a.x_out, c_lo, a.levels);
 }

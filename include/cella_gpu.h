@@ -196,17 +196,20 @@ int cg_timed_iterate(cg_sim* sim, double ms[4]);
  * compute_2048.wgsl:57-84).  Each phase has up to CG_MAX_VARIANTS variants:
  *   0-2  CTA shapes (rows per CTA and threads for the row FFTs, columns per
  *        CTA and threads for the column pass, tile rows and columns per
- *        thread for diffusion), radix-16 plans; bit-identical results.
- *        The forward row FFT's variant 2 is variant 1's tile in a
- *        persistent grid whose CTAs bring each block of rows in with one
- *        bulk copy, the next block's during the current one's transform.
+ *        thread for diffusion), radix-16 plans; bit-identical results.  0,
+ *        which an untuned world runs, is the shape that measured best at
+ *        the grid side.  From side 1024 on the forward row FFT's variant 2
+ *        is variant 1's tile in a persistent grid whose CTAs bring each
+ *        block of rows in with one bulk copy, the next block's during the
+ *        current one's transform, and diffusion's variant 0 takes 16- or
+ *        8-row strips (variant 1 or 3) by the world's size.
  *   3    for diffusion, at every grid side: variant 1's register tiles in
  *        strips of 8 rows instead of 16; bit-identical results.
  *   3, 4 FFT plans, for the row and column phases at grid sides >= 512:
  *        row FFTs over two real rows as one complex sequence of length n
  *        with radix-16 (3) or radix-8 (4) passes; the column pass with its
  *        forward and inverse plan orders swapped (remainder-first radix
- *        first forward) in the CTA shape of variant 1 (3) or 0 (4).  These
+ *        first forward) in the CTA shape of variant 0 (3) or 1 (4).  These
  *        agree with variants 0-2 to rounding (the same step error bar
  *        against FP64), not bit for bit.
  * Diffusion has variants 0-3; the other phases below side 512 have 0-2.
@@ -223,8 +226,9 @@ int cg_autotune(cg_sim* sim, int reps, double ms_out[4 * CG_MAX_VARIANTS], int c
  * CG_ERR_ARG.  Setting re-captures the graphs. */
 int cg_set_variants(cg_sim* sim, const int v[4]);
 /* Layout of the step graphs: 0, each channel's launches on a forked stream of
- * its own, so the channels' phases overlap; 1, one stream with one launch
- * per phase over all channels.  Both compute the same bits; after the
+ * its own, so the channels' phases overlap (from side 512 on: below it a
+ * launch is shorter than the forks and joins, and 0 is the same as 1); 1, one
+ * stream with one launch per phase over all channels.  Both compute the same bits; after the
  * variants, cg_autotune times both (graphs of steps that all read the
  * current state, so the world does not advance) and keeps the faster.
  * Setting re-captures the graphs. */
