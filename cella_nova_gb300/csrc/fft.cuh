@@ -38,8 +38,15 @@ struct SmemRows {
 template <class F>
 struct is_smem_rows : std::is_same<std::remove_cv_t<std::remove_reference_t<F>>, SmemRows> {};
 
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// Complex sums as one packed FP32 instruction each (two roundings, the bits of
+// two scalar sums; the product by -1 in the difference is exact).  The
+// butterflies are mostly these: it freed 6-8 registers in the column pass and
+// took the inverse row pass from 52.6 to 50.1 us at 2048^2 and from 15.3 to
+// 14.7 us at 1024^2 (C=3, K=9, variant 3).
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+    return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+}
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
