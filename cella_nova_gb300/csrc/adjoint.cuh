@@ -273,21 +273,35 @@ __global__ void __launch_bounds__(GrowthRows<LOGN, V>::RT, 512 / GrowthRows<LOGN
 //    (column 0: P conj(alpha) + conj P(-ky) conj(beta)), then one inverse
 //    column FFT, written over the row spectra of c.
 // ---------------------------------------------------------------------------
-template <int LOGN, int V = 0>
+// Tiles arrive by bulk copies as in the forward pass.  At small sides the
+// U tiles (after that of x) and the spectrum tiles have a staging buffer and
+// an mbarrier each, so the next tile of either kind lands during this one's
+// work, and start() (the wait for the kernel before this one) comes after
+// the first spectrum tile's issue; at larger sides they share one buffer.
+// The CTA of column 0 has its own form of the products (below); the others
+// test nothing per value.  It reads the beta column (row M of the packed
+// spectrum) from global memory: brought into L1 before the column FFT and
+// read a butterfly at a time, because one load at a time made this CTA the
+// length of the kernel (256^2, C=3, K=9: 37 us, of which 12 us per kernel in
+// these loads).
+template <int LOGN, int V = 0, class START>
 __device__ __forceinline__ bool col_conv_adj_body(float2* __restrict__ rowspec,
                                                   const float2* __restrict__ kspec,
                                                   const float2* __restrict__ U,
                                                   float2* __restrict__ kgrad,
                                                   const float2* __restrict__ tw,
                                                   const KernelGroups& groups, int c, int kx0,
-                                                  float2* sm, uint64_t* barp, uint32_t& phase,
-                                                  int* err) {
+                                                  float2* sm, uint64_t* barp, int* err,
+                                                  START start) {
     using G = Geo<LOGN, V>;
-    constexpr int N = G::N, M = G::M, TW = G::TW, T = G::CT;
+    constexpr int N = G::N, M = G::M, TW = G::TW, T = G::CT, NBUF = G::NBUF;
     float2* W = sm;
-    float2* KS = sm + G::KSOFF;
+    float2* KU = sm + G::KSOFF;                  // staging tile of x and U
+    float2* KS = KU + (NBUF - 1) * (TW * N);     // staging tile of the spectra
     float2* Wx = KS + TW * N;   // with kgrad: colFFT of this channel's row spectra
-    uint64_t& bar = *barp;
+    uint64_t* const bar_u = barp;
+    uint64_t* const bar_k = barp + (NBUF - 1);
+    uint32_t done_u = 0, done_k = 0;             // tiles waited for (one count if NBUF = 1)
     const int cnt = groups.in_count[c], base = groups.in_start[c];
     float2* dst = rowspec + (size_t(c) * M + kx0) * N;
     constexpr uint32_t kTileBytes = uint32_t(TW) * N * sizeof(float2);
@@ -300,34 +314,62 @@ __device__ __forceinline__ bool col_conv_adj_body(float2* __restrict__ rowspec,
 #pragma unroll
         for (int r = 0; r < RL; ++r) acc[it][r] = make_float2(0.f, 0.f);
 
-    auto issue = [&](const float2* src) {
+    auto copy = [&](float2* to, const float2* src, uint64_t* bar) {
+        if (threadIdx.x == 0) {
+            mbar_arrive_expect_tx(bar, kTileBytes);
+            bulk_g2s(to, src, kTileBytes, bar);
+        }
+    };
+    auto release = [&]() {   // the reads of a staging tile are done: it may be refilled
         fence_proxy_async_smem();
         __syncthreads();
-        if (threadIdx.x == 0) {
-            mbar_arrive_expect_tx(&bar, kTileBytes);
-            bulk_g2s(KS, src, kTileBytes, &bar);
-        }
     };
-    auto wait_tile = [&]() -> bool {
-        const bool ok = mbar_wait(&bar, phase & 1, err);
+    auto u_tile = [&](int gi) { return U + (size_t(groups.in_idx[base + gi]) * M + kx0) * N; };
+    auto k_tile = [&](int gi) {
+        return kspec + (size_t(groups.in_idx[base + gi]) * (M + 1) + kx0) * N;
+    };
+    // pending: a copy of the other kind is in flight (NBUF = 2)
+    auto wait_tile = [&](uint64_t* bar, uint32_t& done, uint64_t* other, uint32_t other_done,
+                         bool pending) -> bool {
+        const bool ok = mbar_wait(bar, done & 1, err);
         if (__syncthreads_or(!ok)) {
-            mbar_wait(&bar, phase & 1, nullptr);
+            mbar_wait(bar, done & 1, nullptr);
+            if (NBUF == 2 && pending) mbar_wait(other, other_done & 1, nullptr);
             return false;
         }
-        ++phase;
+        ++done;
         return true;
     };
-    auto ld_in = [&](int s, int i, int, int) { return KS[s * N + i]; };
+    auto wait_u = [&](bool pending) {
+        return wait_tile(bar_u, done_u, bar_k, done_k, pending);
+    };
+    auto wait_k = [&](bool pending) {
+        if constexpr (NBUF == 1) return wait_tile(bar_u, done_u, nullptr, 0, false);
+        else return wait_tile(bar_k, done_k, bar_u, done_u, pending);
+    };
+    release();
+    if (NBUF == 2 && cnt > 0) copy(KS, k_tile(0), bar_k);
+    start();
+    if (kgrad) copy(KU, dst, bar_u);
+    else if (cnt > 0) copy(KU, u_tile(0), bar_u);
+    auto ld_in = [&](int s, int i, int, int) { return KU[s * N + i]; };
     SmemRows wrows{W, G::CP};
     if (kgrad) {   // X = colFFT(row spectra of x), read before dst is overwritten
-        issue(dst);
-        if (!wait_tile()) return false;
+        if (!wait_u(cnt > 0)) return false;
         SmemRows xrows{Wx, G::CP};
-        FftPasses<N, 1, false, T, TW, false>::run(ld_in, xrows, xrows, xrows, tw + G::TW_COL_FWD);
+        fft_with_hook<N, false, T, TW, false>(ld_in, xrows, xrows, xrows, tw + G::TW_COL_FWD,
+                                              [&]() {
+                                                  if (cnt > 0) {
+                                                      release();
+                                                      copy(KU, u_tile(0), bar_u);
+                                                  }
+                                              });
     }
 
     for (int gi = 0; gi < cnt; ++gi) {
         const int k = groups.in_idx[base + gi];
+        const float2* kb = kspec + (size_t(k) * (M + 1) + M) * N;
+        if (kx0 == 0) warm_table<T>(kb, N);
         float2* kg = kgrad ? kgrad + (size_t(k) * M + kx0) * N : nullptr;
         // this thread's kernel-gradient values, loaded now so that they land
         // during the column FFT below (only this CTA touches them)
@@ -343,55 +385,73 @@ __device__ __forceinline__ bool col_conv_adj_body(float2* __restrict__ rowspec,
                 }
             }
         }
-        issue(U + (size_t(k) * M + kx0) * N);
-        if (!wait_tile()) return false;
-        const float2* ktile = kspec + (size_t(k) * (M + 1) + kx0) * N;
+        if (!wait_u(true)) return false;
         fft_with_hook<N, false, T, TW, false>(ld_in, wrows, wrows, wrows, tw + G::TW_COL_FWD,
-                                             [&]() { issue(ktile); });
-        if (!wait_tile()) return false;
-        const float2* kb = kspec + (size_t(k) * (M + 1) + M) * N;
+                                              [&]() {
+                                                  release();
+                                                  if (NBUF == 1) copy(KS, k_tile(gi), bar_k);
+                                                  else if (gi + 1 < cnt) copy(KU, u_tile(gi + 1), bar_u);
+                                              });
+        if (!wait_k(gi + 1 < cnt)) return false;
+        auto products = [&](auto col0) {
+            constexpr bool C0 = decltype(col0)::value;
 #pragma unroll
-        for (int it = 0; it < IPTL; ++it) {
-            const int item = threadIdx.x + it * T;
-            if ((TW * JL) % T == 0 || item < TW * JL) {
-                const int s = item / JL, j = item % JL;
+            for (int it = 0; it < IPTL; ++it) {
+                const int item = threadIdx.x + it * T;
+                if ((TW * JL) % T == 0 || item < TW * JL) {
+                    const int s = item / JL, j = item % JL;
+                    float2 kbv[RL];
+                    if constexpr (C0) {
+                        if (s == 0)
 #pragma unroll
-                for (int r = 0; r < RL; ++r) {
-                    const int i = j + r * JL;
-                    const float2 p = W[s * G::CP + pidx(i)];
-                    float2 g = cmulc(p, KS[s * N + i]);
-                    float2 pm;
-                    if (kx0 + s == 0) {
-                        pm = cconj(W[pidx((N - i) & (N - 1))]);
-                        g = cadd(g, cmulc(pm, __ldg(&kb[i])));
+                            for (int r = 0; r < RL; ++r) kbv[r] = __ldg(&kb[j + r * JL]);
                     }
-                    acc[it][r] = cadd(acc[it][r], g);
-                    if (kg) {
-                        // kgrad_k += colFFT(ubar_k) conj(X); column 0 carries the
-                        // kx = 0 and kx = n/2 spectra (FA = (P + conj P(-)) / 2,
-                        // FB = (P - conj P(-)) / (2i)) and stores FA conj(XA) +
-                        // i FB conj(XB)
-                        const float2 px = Wx[s * G::CP + pidx(i)];
-                        float2 v;
-                        if (kx0 + s == 0) {
-                            const float2 pxm = cconj(Wx[pidx((N - i) & (N - 1))]);
-                            const float2 au = make_float2(0.5f * (p.x + pm.x), 0.5f * (p.y + pm.y));
-                            const float2 du = make_float2(0.5f * (p.x - pm.x), 0.5f * (p.y - pm.y));
-                            const float2 bu = make_float2(du.y, -du.x);
-                            const float2 ax = make_float2(0.5f * (px.x + pxm.x), 0.5f * (px.y + pxm.y));
-                            const float2 dx = make_float2(0.5f * (px.x - pxm.x), 0.5f * (px.y - pxm.y));
-                            const float2 bx = make_float2(dx.y, -dx.x);
-                            const float2 g0 = cmulc(au, ax), gm = cmulc(bu, bx);
-                            v = make_float2(g0.x - gm.y, g0.y + gm.x);   // g0 + i gm
-                        } else {
-                            v = cmulc(p, px);
+#pragma unroll
+                    for (int r = 0; r < RL; ++r) {
+                        const int i = j + r * JL;
+                        const float2 p = W[s * G::CP + pidx(i)];
+                        float2 g = cmulc(p, KS[s * N + i]);
+                        float2 pm;
+                        if (C0 && s == 0) {
+                            pm = cconj(W[pidx((N - i) & (N - 1))]);
+                            g = cadd(g, cmulc(pm, kbv[r]));
                         }
-                        kg[size_t(s) * N + i] = cadd(kgv[it][r], v);
+                        acc[it][r] = cadd(acc[it][r], g);
+                        if (kg) {
+                            // kgrad_k += colFFT(ubar_k) conj(X); column 0 carries the
+                            // kx = 0 and kx = n/2 spectra (FA = (P + conj P(-)) / 2,
+                            // FB = (P - conj P(-)) / (2i)) and stores FA conj(XA) +
+                            // i FB conj(XB)
+                            const float2 px = Wx[s * G::CP + pidx(i)];
+                            float2 v;
+                            if (C0 && s == 0) {
+                                const float2 pxm = cconj(Wx[pidx((N - i) & (N - 1))]);
+                                const float2 au = make_float2(0.5f * (p.x + pm.x), 0.5f * (p.y + pm.y));
+                                const float2 du = make_float2(0.5f * (p.x - pm.x), 0.5f * (p.y - pm.y));
+                                const float2 bu = make_float2(du.y, -du.x);
+                                const float2 ax = make_float2(0.5f * (px.x + pxm.x), 0.5f * (px.y + pxm.y));
+                                const float2 dx = make_float2(0.5f * (px.x - pxm.x), 0.5f * (px.y - pxm.y));
+                                const float2 bx = make_float2(dx.y, -dx.x);
+                                const float2 g0 = cmulc(au, ax), gm = cmulc(bu, bx);
+                                v = make_float2(g0.x - gm.y, g0.y + gm.x);   // g0 + i gm
+                            } else {
+                                v = cmulc(p, px);
+                            }
+                            kg[size_t(s) * N + i] = cadd(kgv[it][r], v);
+                        }
                     }
                 }
             }
+        };
+        if (kx0 == 0)
+            products(std::true_type{});
+        else
+            products(std::false_type{});
+        release();
+        if (gi + 1 < cnt) {
+            if (NBUF == 1) copy(KU, u_tile(gi + 1), bar_u);
+            else copy(KS, k_tile(gi + 1), bar_k);
         }
-        __syncthreads();
     }
     auto ld_acc = [&](int, int, int it, int r) { return acc[it][r]; };
     auto gst = [&](int s, int i, float2 v, int, int) { dst[size_t(s) * N + i] = v; };
@@ -407,8 +467,10 @@ struct AdjColGeo {
         Geo<LOGN, V>::COL_SMEM + size_t(Geo<LOGN, V>::TW) * Geo<LOGN, V>::CP * sizeof(float2);
 };
 
+// (small sides: registers before resident CTAs, which the grid does not fill)
 template <int LOGN, int V = 0>
-__global__ void __launch_bounds__(Geo<LOGN, V>::CT, 512 / Geo<LOGN, V>::CT) k_col_conv_adj(float2* __restrict__ rowspec,
+__global__ void __launch_bounds__(Geo<LOGN, V>::CT,
+                                  (Geo<LOGN, V>::SMALL ? 256 : 512) / Geo<LOGN, V>::CT) k_col_conv_adj(float2* __restrict__ rowspec,
                                                           const float2* __restrict__ kspec,
                                                           const float2* __restrict__ U,
                                                           float2* __restrict__ kgrad,
@@ -416,13 +478,16 @@ __global__ void __launch_bounds__(Geo<LOGN, V>::CT, 512 / Geo<LOGN, V>::CT) k_co
                                                           const __grid_constant__ KernelGroups groups,
                                                           int* err) {
     extern __shared__ __align__(128) float2 sm_cadj[];
-    __shared__ __align__(8) uint64_t bar;
-    pdl_wait();
-    pdl_launch_dependents();
-    init_tile_barrier(&bar);
-    uint32_t phase = 0;
+    using G = Geo<LOGN, V>;
+    __shared__ __align__(8) uint64_t bar[G::NBUF];
+    init_tile_barriers<G::NBUF>(bar);
+    if constexpr (G::SMALL)
+        warm_table<G::CT>(tw + G::TW_COL_FWD, tw_size(G::N, false) + tw_size(G::N, true));
     col_conv_adj_body<LOGN, V>(rowspec, kspec, U, kgrad, tw, groups, blockIdx.y,
-                            blockIdx.x * Geo<LOGN, V>::TW, sm_cadj, &bar, phase, err);
+                               blockIdx.x * G::TW, sm_cadj, bar, err, [] {
+                                   pdl_wait();
+                                   pdl_launch_dependents();
+                               });
 }
 
 // ---------------------------------------------------------------------------
