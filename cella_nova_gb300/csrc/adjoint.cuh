@@ -31,17 +31,45 @@ namespace cg {
 
 
 // ---------------------------------------------------------------------------
-// 2. Diffusion backward (one channel tile per CTA, 256 threads).
+// 2. Diffusion backward (one channel tile per CTA).
 // ---------------------------------------------------------------------------
 // A and ybar (2-pixel halo) and the state (1-pixel halo) arrive by 16-byte
 // loads: their tiles reach 4 pixels past the tile on each side, so every
 // load stays aligned (n is a multiple of 4, also across the toroidal wrap).
+
+// Division of several numerators by one z, each correctly rounded as x / z
+// is: from the correctly rounded reciprocal r of z, q0 = fl(x r) is within an
+// ulp of x / z, and q0 + (x - q0 z) r with the exact remainder is its rounding
+// (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34 (1990) 111-119).  One
+// reciprocal and three instructions per numerator instead of a division each.
+// Outside [2^-100, 2^100], where r or the remainder could leave the normal
+// range, it divides.
+struct Divisor {
+    float z, r;
+    bool plain;
+    __device__ __forceinline__ explicit Divisor(float d) : z(d) {
+        const float m = fabsf(d);
+        plain = !(m >= 7.8886091e-31f && m <= 1.2676506e30f);
+        r = __frcp_rn(d);
+    }
+    __device__ __forceinline__ float divide(float x) const {
+        if (plain) return x / z;
+        const float q0 = x * r;
+        return fmaf(fmaf(-q0, z, x), r, q0);
+    }
+};
+
 template <int LOGN, int V = 0>
 struct DiffBwdGeo {
     static constexpr int TX = Geo<LOGN, V>::TX, TY = Geo<LOGN, V>::TY;
     static constexpr int AS = TX + 8, AH = TY + 4, HW = TX + 2, QH = TY + 2, V4 = AS / 4;
+    static constexpr int NSEG = 4;                     // row segments of a halo column
+    static constexpr int ZR = (QH + NSEG - 1) / NSEG;  // rows per segment, at most
+    static constexpr int NOUT = 4, OR = TY / NOUT;     // row segments of an output column
+    static constexpr int THREADS = (HW * NSEG + 31) / 32 * 32;
     static constexpr size_t SMEM = size_t(2 * AH * AS + QH * AS + 2 * QH * HW) * sizeof(float);
-    static_assert(TX % 4 == 0, "tile shape");
+    static_assert(TX % 4 == 0 && TY % NOUT == 0, "tile shape");
 };
 
 template <int LOGN, int V = 0>
@@ -75,43 +103,81 @@ __device__ __forceinline__ void diffusion_bwd_body(const float* __restrict__ A,
                 Xp + size_t((y0 + r - 1) & (N - 1)) * N + cx));
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < QH * HW; i += blockDim.x) {
-        const int r = i / HW, q = i % HW;
-        float z = 0.f, qb = 0.f;
-#pragma unroll
-        for (int di = 0; di < 3; ++di)
+    // Down a halo column: the three columns of A and ybar around it, three
+    // rows of each in registers (slots by row modulo 3), so a position reads
+    // six values from shared memory instead of eighteen; every sum keeps its
+    // order, row by row from the top left.
+    const int t = threadIdx.x;
+    if (t < HW * D::NSEG) {
+        const int q = t % HW, seg = t / HW;
+        const int r0 = seg * QH / D::NSEG, rn = (seg + 1) * QH / D::NSEG - r0;
+        float a[3][3], y[3][3];
+        auto load = [&](int slot, int r) {
 #pragma unroll
             for (int dj = 0; dj < 3; ++dj) {
-                const float a = sA[r + di][q + dj + 2];
-                z += a;
-                qb = fmaf(sY[r + di][q + dj + 2], a, qb);
+                a[slot][dj] = sA[r][q + dj + 2];
+                y[slot][dj] = sY[r][q + dj + 2];
             }
-        const int gy = (y0 + r - 1) & (N - 1), gx = (x0 + q - 1) & (N - 1);
-        const float xv = sX[r][q + 3];
-        const float qv = xv / z;
-        sQ[r][q] = qv;
-        sZb[r][q] = -qb * qv / z;
-        if (r >= 1 && r <= TY && q >= 1 && q <= TX) xbar[plane + size_t(gy) * N + gx] = qb / z;
+        };
+        load(0, r0);
+        load(1, r0 + 1);
+        const bool inner = q >= 1 && q <= TX;
+        float* xb = xbar + plane + size_t(y0) * N + x0 + (q - 1);
+#pragma unroll
+        for (int i = 0; i < D::ZR; ++i) {
+            if (i >= rn) break;
+            const int r = r0 + i;
+            load((i + 2) % 3, r + 2);
+            float z = 0.f, qb = 0.f;
+#pragma unroll
+            for (int di = 0; di < 3; ++di)
+#pragma unroll
+                for (int dj = 0; dj < 3; ++dj) {
+                    const float av = a[(i + di) % 3][dj];
+                    z += av;
+                    qb = fmaf(y[(i + di) % 3][dj], av, qb);
+                }
+            const Divisor by(z);
+            const float qv = by.divide(sX[r][q + 3]);
+            sQ[r][q] = qv;
+            sZb[r][q] = by.divide(-qb * qv);
+            if (inner && r >= 1 && r <= TY) xb[(r - 1) * N] = by.divide(qb);
+        }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < TY * TX; i += blockDim.x) {
-        const int r = i / TX, q = i % TX;
-        float P = 0.f, SZ = 0.f;
-#pragma unroll
-        for (int di = 0; di < 3; ++di)
+    if (t < TX * D::NOUT) {
+        const int q = t % TX, r0 = (t / TX) * D::OR;
+        float qs[3][3], zs[3][3];
+        auto load = [&](int slot, int r) {
 #pragma unroll
             for (int dj = 0; dj < 3; ++dj) {
-                P += sQ[r + di][q + dj];
-                SZ += sZb[r + di][q + dj];
+                qs[slot][dj] = sQ[r][q + dj];
+                zs[slot][dj] = sZb[r][q + dj];
             }
-        const float a = sA[r + 2][q + 4];
-        const float Ab = fmaf(sY[r + 2][q + 4], P, SZ);
-        abar[plane + size_t(y0 + r) * N + x0 + q] = temp * a * Ab;
+        };
+        load(0, r0);
+        load(1, r0 + 1);
+        float* ab = abar + plane + size_t(y0 + r0) * N + x0 + q;
+#pragma unroll
+        for (int i = 0; i < D::OR; ++i) {
+            load((i + 2) % 3, r0 + i + 2);
+            float P = 0.f, SZ = 0.f;
+#pragma unroll
+            for (int di = 0; di < 3; ++di)
+#pragma unroll
+                for (int dj = 0; dj < 3; ++dj) {
+                    P += qs[(i + di) % 3][dj];
+                    SZ += zs[(i + di) % 3][dj];
+                }
+            const float a = sA[r0 + i + 2][q + 4];
+            const float Ab = fmaf(sY[r0 + i + 2][q + 4], P, SZ);
+            ab[i * N] = temp * a * Ab;
+        }
     }
 }
 
 template <int LOGN, int V = 0>
-__global__ void __launch_bounds__(256) k_diffusion_bwd(const float* __restrict__ A,
+__global__ void __launch_bounds__(DiffBwdGeo<LOGN, V>::THREADS) k_diffusion_bwd(const float* __restrict__ A,
                                                         const float* __restrict__ x,
                                                         const float* __restrict__ ybar,
                                                         float* __restrict__ xbar,
@@ -576,7 +642,8 @@ constexpr int kDiffBwdVariant = 1;
 template <int LOGN, int V>
 cudaError_t launch_diff_bwd(const BwdArgs& a, cudaStream_t st) {
     using G = Geo<LOGN, V>;
-    return launch_pdl(k_diffusion_bwd<LOGN, V>, dim3(G::N / G::TX, G::N / G::TY, a.C), 256,
+    return launch_pdl(k_diffusion_bwd<LOGN, V>, dim3(G::N / G::TX, G::N / G::TY, a.C),
+                      DiffBwdGeo<LOGN, V>::THREADS,
                       DiffBwdGeo<LOGN, V>::SMEM, st, a.A, a.x, a.ybar, a.xbar, a.abar, a.temp);
 }
 template <int LOGN, int V>
