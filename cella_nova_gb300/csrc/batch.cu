@@ -237,6 +237,7 @@ struct cg_batch {
         float2* kspec = nullptr;
         float* kspec_re = nullptr;
         std::vector<uint8_t> kreal;   // per kernel: point-symmetric (cg_batch_set_kernel)
+        std::vector<uint8_t> kset;    // per kernel: uploaded
         float2* U = nullptr;
         float* A = nullptr;
         KernelGroups groups{};
@@ -269,9 +270,12 @@ struct cg_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     bool kreal_all = false;   // every world's kernels point-symmetric: real column pass
+    // the step graphs exist: captured with the last kernel's first upload, or
+    // with the first step
+    bool graphs_ready = false;
     int cur = 0;
     int device = 0;
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph[2][2] = {};   // kBatchGraphSteps[i] steps, per parity
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     size_t max_px = 0;
 };
@@ -281,8 +285,9 @@ namespace {
 void batch_release(cg_batch* b) {
     if (!b) return;
     cudaSetDevice(b->device);
-    for (auto& g : b->graph)
-        if (g) cudaGraphExecDestroy(g);
+    for (auto& per_parity : b->graph)
+        for (auto& g : per_parity)
+            if (g) cudaGraphExecDestroy(g);
     for (auto& e : b->ev)
         if (e) cudaEventDestroy(e);
     for (auto& w : b->worlds) {
@@ -376,10 +381,16 @@ StepArgs world_step_args(const cg_batch* b, int w, int parity, const Variants& v
     return a;
 }
 
-// Streams and events one class step in mode 1 uses: kLanes lane groups of
+// Steps per graph of cg_batch_step.  Worlds share no data, so within a graph
+// each size class (and in mode 1 each world) goes through its steps without
+// waiting for the others; they meet where the graph ends.
+constexpr int kBatchGraphSteps[2] = {4, 1};
+constexpr int kOneBatchStep = 1;   // index of the one-step graph
+
+// Streams and events the class steps in mode 1 use: kLanes lane groups of
 // C_max streams (world i of the class runs on lane group i % kLanes, channel
 // c on its stream c), a join event per lane stream and, per world and
-// channel, the event after its column pass.
+// channel, the events after its column pass and its inverse row pass.
 constexpr int kLanes = 8;
 struct LanePool {
     std::vector<cudaStream_t> streams;   // [kLanes][cmax]
@@ -416,19 +427,24 @@ int class_cmax(const cg_batch* b, const cg_batch::SizeClass& sc) {
 int class_events(const cg_batch* b, const cg_batch::SizeClass& sc) {
     int n = 1 + kLanes * class_cmax(b, sc);
     for (const auto& W : b->worlds)
-        if (W.logn == sc.logn) n += W.C;
+        if (W.logn == sc.logn) n += 2 * W.C;
     return n;
 }
 
-// One step of one class on stream st, after what st holds and before what
+// nsteps steps of one class on stream st, after what st holds and before what
 // it gets next (the lanes fork from st and join back into it).
-cudaError_t enqueue_class_step(cg_batch* b, const cg_batch::SizeClass& sc, int parity,
-                               cudaStream_t st, LanePool* pool) {
+// fixed_parity: every step reads the state of `parity` and writes the other
+// buffer (the tuner's timing: replaying advances nothing).
+cudaError_t enqueue_class_steps(cg_batch* b, const cg_batch::SizeClass& sc, int parity,
+                                int nsteps, cudaStream_t st, LanePool* pool,
+                                bool fixed_parity = false) {
+    auto parity_at = [&](int t) { return fixed_parity ? parity : parity ^ (t & 1); };
     if (sc.mode == 0) {
-        for (int ph = 0; ph < 4; ++ph) {
-            cudaError_t e = launch_class_phase(b, sc, ph, sc.var[ph], parity, st);
-            if (e != cudaSuccess) return e;
-        }
+        for (int t = 0; t < nsteps; ++t)
+            for (int ph = 0; ph < 4; ++ph) {
+                cudaError_t e = launch_class_phase(b, sc, ph, sc.var[ph], parity_at(t), st);
+                if (e != cudaSuccess) return e;
+            }
         return cudaSuccess;
     }
     Variants var;
@@ -446,20 +462,30 @@ cudaError_t enqueue_class_step(cg_batch* b, const cg_batch::SizeClass& sc, int p
     for (int w = 0; w < int(b->worlds.size()) && e == cudaSuccess; ++w) {
         const auto& W = b->worlds[size_t(w)];
         if (W.logn != sc.logn) continue;
-        const StepArgs a = world_step_args(b, w, parity, var);
         cudaStream_t* ls = &pool->streams[size_t(i % kLanes) * pool->cmax];
         ++i;
-        const size_t ev0 = ev;
-        for (int c = 0; c < W.C && e == cudaSuccess; ++c) {
-            e = ops->step_channel(a, kPhaseRowFwd | kPhaseColConv, c, ls[c]);
-            if (e == cudaSuccess) e = cudaEventRecord(pool->events[ev0 + c], ls[c]);
-        }
-        ev += size_t(W.C);
-        // a channel's inverse row pass reads U of every input channel
-        for (int c = 0; c < W.C && e == cudaSuccess; ++c) {
-            for (int o = 0; o < W.C && e == cudaSuccess; ++o)
-                if (o != c) e = cudaStreamWaitEvent(ls[c], pool->events[ev0 + o], 0);
-            if (e == cudaSuccess) e = ops->step_channel(a, kPhaseGrowth | kPhaseDiffusion, c, ls[c]);
+        cudaEvent_t* ecol = &pool->events[ev];
+        cudaEvent_t* ec2r = ecol + W.C;
+        ev += 2 * size_t(W.C);
+        for (int t = 0; t < nsteps && e == cudaSuccess; ++t) {
+            const StepArgs a = world_step_args(b, w, parity_at(t), var);
+            for (int c = 0; c < W.C && e == cudaSuccess; ++c) {
+                e = ops->step_channel(a, kPhaseRowFwd, c, ls[c]);
+                // a column pass overwrites U, which every channel's inverse
+                // row pass of the step before read
+                for (int o = 0; t > 0 && o < W.C && e == cudaSuccess; ++o)
+                    if (o != c) e = cudaStreamWaitEvent(ls[c], ec2r[o], 0);
+                if (e == cudaSuccess) e = ops->step_channel(a, kPhaseColConv, c, ls[c]);
+                if (e == cudaSuccess) e = cudaEventRecord(ecol[c], ls[c]);
+            }
+            // a channel's inverse row pass reads U of every input channel
+            for (int c = 0; c < W.C && e == cudaSuccess; ++c) {
+                for (int o = 0; o < W.C && e == cudaSuccess; ++o)
+                    if (o != c) e = cudaStreamWaitEvent(ls[c], ecol[o], 0);
+                if (e == cudaSuccess) e = ops->step_channel(a, kPhaseGrowth, c, ls[c]);
+                if (e == cudaSuccess) e = cudaEventRecord(ec2r[c], ls[c]);
+                if (e == cudaSuccess) e = ops->step_channel(a, kPhaseDiffusion, c, ls[c]);
+            }
         }
     }
     for (auto lane : pool->streams) {
@@ -471,15 +497,18 @@ cudaError_t enqueue_class_step(cg_batch* b, const cg_batch::SizeClass& sc, int p
     return e;
 }
 
-// One graph per ping-pong parity, (re)captured from the current variants.
-// The size classes share no data, so each runs its four phases on a forked
-// stream of its own: one class's phase tails overlap the other's work.
+// One graph per step count and ping-pong parity, (re)captured from the
+// current variants.  The size classes share no data, so each runs its steps
+// on a forked stream of its own: one class's phase tails overlap the other's
+// work.
 cudaError_t capture_batch_graphs(cg_batch* b) {
-    for (auto& g : b->graph)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
+    b->graphs_ready = false;
+    for (auto& per_parity : b->graph)
+        for (auto& g : per_parity)
+            if (g) {
+                cudaGraphExecDestroy(g);
+                g = nullptr;
+            }
     const size_t nc = b->classes.size();
     std::vector<cudaStream_t> st(nc, nullptr);
     std::vector<cudaEvent_t> done(nc, nullptr);
@@ -492,7 +521,8 @@ cudaError_t capture_batch_graphs(cg_batch* b) {
         if (e == cudaSuccess && b->classes[i].mode == 1)
             e = pools[i].make(class_cmax(b, b->classes[i]), class_events(b, b->classes[i]));
     }
-    for (int p = 0; p < 2 && e == cudaSuccess; ++p) {
+    for (int q = 0; q < 4 && e == cudaSuccess; ++q) {
+        const int p = q & 1, steps = kBatchGraphSteps[q >> 1];
         cudaGraph_t g = nullptr;
         e = cudaStreamBeginCapture(st[0], cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
@@ -500,7 +530,7 @@ cudaError_t capture_batch_graphs(cg_batch* b) {
             for (size_t i = 1; i < nc && le == cudaSuccess; ++i)
                 le = cudaStreamWaitEvent(st[i], fork, 0);
             for (size_t i = 0; i < nc && le == cudaSuccess; ++i)
-                le = enqueue_class_step(b, b->classes[i], p, st[i], &pools[i]);
+                le = enqueue_class_steps(b, b->classes[i], p, steps, st[i], &pools[i]);
             for (size_t i = 1; i < nc && le == cudaSuccess; ++i) {
                 le = cudaEventRecord(done[i], st[i]);
                 if (le == cudaSuccess) le = cudaStreamWaitEvent(st[0], done[i], 0);
@@ -509,7 +539,7 @@ cudaError_t capture_batch_graphs(cg_batch* b) {
             e = cudaStreamEndCapture(st[0], &g);
             if (le != cudaSuccess) e = le;
         }
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph[p], g, 0);
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph[q >> 1][p], g, 0);
         if (g) cudaGraphDestroy(g);
     }
     for (size_t i = 0; i < nc; ++i) {
@@ -517,17 +547,23 @@ cudaError_t capture_batch_graphs(cg_batch* b) {
         if (done[i]) cudaEventDestroy(done[i]);
     }
     if (fork) cudaEventDestroy(fork);
+    b->graphs_ready = e == cudaSuccess;
     return e;
+}
+
+// Capture the step graphs anew, if they have been captured at all.
+cudaError_t recapture_batch(cg_batch* b) {
+    return b->graphs_ready ? capture_batch_graphs(b) : cudaSuccess;
 }
 
 // Device ms of one whole batched step (every side, as captured), averaged
 // over reps launches of the step graph of the current parity: each launch
 // reads the current state and writes the spare buffer, so nothing steps.
 int time_batch_step(cg_batch* b, int reps, double* ms) {
-    cudaError_t e = cudaGraphLaunch(b->graph[b->cur], b->stream);   // warm-up
+    cudaGraphExec_t ge = b->graph[kOneBatchStep][b->cur];
+    cudaError_t e = cudaGraphLaunch(ge, b->stream);   // warm-up
     if (e == cudaSuccess) e = cudaEventRecord(b->ev[0], b->stream);
-    for (int r = 0; r < reps && e == cudaSuccess; ++r)
-        e = cudaGraphLaunch(b->graph[b->cur], b->stream);
+    for (int r = 0; r < reps && e == cudaSuccess; ++r) e = cudaGraphLaunch(ge, b->stream);
     if (e == cudaSuccess) e = cudaEventRecord(b->ev[1], b->stream);
     if (e == cudaSuccess) e = cudaEventSynchronize(b->ev[1]);
     float f = 0.f;
@@ -538,7 +574,8 @@ int time_batch_step(cg_batch* b, int reps, double* ms) {
 }
 
 // Device ms of one step of class sc alone (its current mode and variants),
-// averaged over reps launches of a captured one-step graph.
+// averaged over reps launches of a captured graph of as many steps as
+// cg_batch_step's longest.
 int time_class_step(cg_batch* b, const cg_batch::SizeClass& sc, int reps, double* ms) {
     cudaStream_t ts = nullptr;
     cudaGraph_t g = nullptr;
@@ -548,7 +585,8 @@ int time_class_step(cg_batch* b, const cg_batch::SizeClass& sc, int reps, double
     if (e == cudaSuccess && sc.mode == 1) e = pool.make(class_cmax(b, sc), class_events(b, sc));
     if (e == cudaSuccess) e = cudaStreamBeginCapture(ts, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        const cudaError_t le = enqueue_class_step(b, sc, b->cur, ts, &pool);
+        const cudaError_t le =
+            enqueue_class_steps(b, sc, b->cur, kBatchGraphSteps[0], ts, &pool, true);
         e = cudaStreamEndCapture(ts, &g);
         if (le != cudaSuccess) e = le;
     }
@@ -564,7 +602,7 @@ int time_class_step(cg_batch* b, const cg_batch::SizeClass& sc, int reps, double
     if (g) cudaGraphDestroy(g);
     if (ts) cudaStreamDestroy(ts);
     if (e != cudaSuccess) return cuda_fail(e, "timing a batched step");
-    *ms = double(f) / reps;
+    *ms = double(f) / reps / kBatchGraphSteps[0];
     return CG_OK;
 }
 
@@ -652,6 +690,7 @@ int cg_batch_create(int n_worlds, const int* n, const int* C, const int* K, cons
         chk(cudaMalloc(&W.kspec, sizeof(float2) * W.K * (half + W.n)), "cudaMalloc(kspec)");
         chk(cudaMalloc(&W.kspec_re, sizeof(float) * W.K * (half + W.n)), "cudaMalloc(kspec_re)");
         W.kreal.assign(size_t(W.K), 0);
+        W.kset.assign(size_t(W.K), 0);
         chk(cudaMalloc(&W.U, sizeof(float2) * W.K * half), "cudaMalloc(U)");
         chk(cudaMalloc(&W.A, sizeof(float) * W.C * px), "cudaMalloc(A)");
         if (rc == CG_OK) {
@@ -761,7 +800,6 @@ int cg_batch_create(int n_worlds, const int* n, const int* C, const int* K, cons
         chk(cudaMalloc(&b->mass_partial, sizeof(double) * kMaxC * kMassBlocks), "cudaMalloc(mass)");
     if (rc == CG_OK) chk(cudaMalloc(&b->mass_out, sizeof(double) * kMaxC), "cudaMalloc(mass)");
     for (int i = 0; i < 5 && rc == CG_OK; ++i) chk(cudaEventCreate(&b->ev[i]), "cudaEventCreate");
-    if (rc == CG_OK) chk(capture_batch_graphs(b), "capturing the batched step graph");
     if (rc == CG_OK) chk(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
     if (rc != CG_OK) {
         batch_release(b);
@@ -806,14 +844,19 @@ int cg_batch_set_kernel(cg_batch* b, int world, int k, const float* spec) {
                                  b->stream),
                "keeping the real parts");
     W.kreal[size_t(k)] = real ? 1 : 0;
-    bool all = true;
-    for (const auto& w : b->worlds)
+    bool all = true, complete = !b->graphs_ready;
+    W.kset[size_t(k)] = 1;
+    for (const auto& w : b->worlds) {
         for (uint8_t r : w.kreal) all = all && r != 0;
-    if (all != b->kreal_all) {
+        for (uint8_t u : w.kset) complete = complete && u != 0;
+    }
+    const bool changed = all != b->kreal_all;
+    if (changed) {
         BCHECK(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
         b->kreal_all = all;
-        BCHECK(capture_batch_graphs(b), "re-capturing the batched step graph");
     }
+    if (complete) BCHECK(capture_batch_graphs(b), "capturing the batched step graph");
+    else if (changed) BCHECK(recapture_batch(b), "re-capturing the batched step graph");
     return CG_OK;
 }
 
@@ -836,10 +879,24 @@ int cg_batch_upload_channel(cg_batch* b, int world, int c, const double* data) {
 int cg_batch_step(cg_batch* b, int nsteps) {
     if (!b) return fail(CG_ERR_ARG, "cg_batch_step: NULL handle");
     if (nsteps < 0) return fail(CG_ERR_ARG, "negative step count %d", nsteps);
-    for (int i = 0; i < nsteps; ++i) {
-        BCHECK(cudaGraphLaunch(b->graph[b->cur], b->stream), "cudaGraphLaunch");
-        b->cur ^= 1;
+    int left = nsteps;
+    if (left > 0 && !b->graphs_ready) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(b->stream, &status) != cudaSuccess) cudaGetLastError();
+        if (status != cudaStreamCaptureStatusActive)
+            BCHECK(capture_batch_graphs(b), "capturing the batched step graph");
+        // into the caller's capture: the phases themselves
+        for (; !b->graphs_ready && left > 0; --left) {
+            for (int p = 0; p < 4; ++p)
+                BCHECK(launch_phase(b, p, b->cur, b->stream), "launching a phase");
+            b->cur ^= 1;
+        }
     }
+    for (int i = 0; i < 2; ++i)
+        for (; left >= kBatchGraphSteps[i]; left -= kBatchGraphSteps[i]) {
+            BCHECK(cudaGraphLaunch(b->graph[i][b->cur], b->stream), "cudaGraphLaunch");
+            b->cur ^= kBatchGraphSteps[i] & 1;
+        }
     return CG_OK;
 }
 
@@ -928,7 +985,7 @@ int cg_batch_set_variants(cg_batch* b, int n, const int v[4]) {
                             v[p], p, phase_variant_count(sc.logn, p) - 1, n);
         BCHECK(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
         for (int p = 0; p < 4; ++p) sc.var[p] = v[p];
-        BCHECK(capture_batch_graphs(b), "re-capturing the batched step graph");
+        BCHECK(recapture_batch(b), "re-capturing the batched step graph");
         return CG_OK;
     }
     return fail(CG_ERR_ARG, "the batch has no world of grid side %d", n);
@@ -941,7 +998,7 @@ int cg_batch_set_mode(cg_batch* b, int n, int mode) {
         if ((1 << sc.logn) != n) continue;
         BCHECK(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
         sc.mode = mode;
-        BCHECK(capture_batch_graphs(b), "re-capturing the batched step graph");
+        BCHECK(recapture_batch(b), "re-capturing the batched step graph");
         return CG_OK;
     }
     return fail(CG_ERR_ARG, "the batch has no world of grid side %d", n);

@@ -227,6 +227,10 @@ struct cg_sim {
     float* kspec_re = nullptr;
     std::vector<uint8_t> kreal;
     bool kreal_all = false;
+    // kernels uploaded so far: with the last one the step graphs are captured
+    // (or with the first step), not at creation and again here
+    std::vector<uint8_t> kset;
+    bool graphs_ready = false;
     float2* U = nullptr;       // two [K][n/2][n] buffers, one per ping-pong parity
     float* A = nullptr;
     float2* tw = nullptr;
@@ -234,8 +238,7 @@ struct cg_sim {
     double* mass_partial = nullptr;
     double* mass_out = nullptr;
     int* err = nullptr;   // device error word written by bounded waits
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};     // one step, per parity
-    cudaGraphExec_t graph8[2] = {nullptr, nullptr};    // kStepsPerGraph steps, per parity
+    cudaGraphExec_t graph[4][2] = {};   // kGraphSteps[i] steps, per parity
     cudaGraphExec_t graphR[2] = {nullptr, nullptr};    // one step that also renders
     unsigned* render = nullptr;   // [n][n] packed 0x00RRGGBB
     unsigned char* levels = nullptr;   // [3][n][n] render levels of a rendering step
@@ -292,10 +295,9 @@ namespace {
 void release(cg_sim* s) {
     if (!s) return;
     cudaSetDevice(s->device);
-    for (auto& g : s->graph)
-        if (g) cudaGraphExecDestroy(g);
-    for (auto& g : s->graph8)
-        if (g) cudaGraphExecDestroy(g);
+    for (auto& per_parity : s->graph)
+        for (auto& g : per_parity)
+            if (g) cudaGraphExecDestroy(g);
     for (auto& g : s->graphR)
         if (g) cudaGraphExecDestroy(g);
     for (auto& e : s->ev)
@@ -337,7 +339,12 @@ void release(cg_sim* s) {
     delete s;
 }
 
-constexpr int kStepsPerGraph = 8;
+// Steps per graph.  Between two graphs the GPU drains and starts again (8-10 us
+// at 512^2 with four channels, against 26 us per step), so a count that is
+// no multiple of eight takes graphs of four and two before single steps.
+constexpr int kGraphSteps[4] = {8, 4, 2, 1};
+constexpr int kStepsPerGraph = kGraphSteps[0];
+constexpr int kOneStep = 3;   // index of the one-step graph
 
 // Capture `nsteps` steps starting at ping-pong parity p0 as one graph whose
 // launches are per channel, on one stream per channel, so that independent
@@ -451,13 +458,26 @@ cudaError_t capture_steps(cg_sim* s, int p0, int nsteps, bool render, cudaGraphE
     return e;
 }
 
+void drop_graphs(cg_sim* s) {
+    for (auto* set : {s->graph[0], s->graph[1], s->graph[2], s->graph[3], s->graphR})
+        for (int p = 0; p < 2; ++p)
+            if (set[p]) {
+                cudaGraphExecDestroy(set[p]);
+                set[p] = nullptr;
+            }
+}
+
 int capture_graphs(cg_sim* s) {
+    s->graphs_ready = false;
+    drop_graphs(s);
     for (int p = 0; p < 2; ++p) {
-        cudaError_t e = capture_steps(s, p, 1, false, &s->graph[p]);
-        if (e == cudaSuccess) e = capture_steps(s, p, kStepsPerGraph, false, &s->graph8[p]);
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; i < 4 && e == cudaSuccess; ++i)
+            e = capture_steps(s, p, kGraphSteps[i], false, &s->graph[i][p]);
         if (e == cudaSuccess) e = capture_steps(s, p, 1, true, &s->graphR[p]);
         if (e != cudaSuccess) return cuda_fail(e, "capturing the step graph");
     }
+    s->graphs_ready = true;
     return CG_OK;
 }
 
@@ -510,14 +530,30 @@ int upload_params(cg_sim* s) {
     return CG_OK;
 }
 
-int recapture(cg_sim* s) {
-    for (auto* set : {s->graph, s->graph8, s->graphR})
-        for (int p = 0; p < 2; ++p)
-            if (set[p]) {
-                cudaGraphExecDestroy(set[p]);
-                set[p] = nullptr;
-            }
-    return capture_graphs(s);
+// Capture the step graphs anew, if they have been captured at all.
+int recapture(cg_sim* s) { return s->graphs_ready ? capture_graphs(s) : CG_OK; }
+
+// The step graphs, before a step is enqueued on st: captured now if they are
+// not yet.  Where st itself is being captured and they are not there, the
+// step's kernels go into that capture instead (*direct).
+int ensure_graphs(cg_sim* s, cudaStream_t st, bool* direct) {
+    *direct = false;
+    if (s->graphs_ready) return CG_OK;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) cudaGetLastError();
+    *direct = status == cudaStreamCaptureStatusActive;
+    return *direct ? CG_OK : capture_graphs(s);
+}
+
+// One step's kernels straight into st (with render: the words as well).
+int step_direct(cg_sim* s, cudaStream_t st, bool render) {
+    StepArgs a = s->args(s->cur, nullptr);
+    if (render) a.levels = s->levels;
+    CG_CHECK(s->ops->step(a, kPhaseAll, st), "launching a step");
+    if (render)
+        CG_CHECK(launch_pack_levels(s->levels, s->C, s->px(), s->render, st), "packing levels");
+    s->cur ^= 1;
+    return CG_OK;
 }
 
 int ensure_backward(cg_sim* s) {
@@ -634,6 +670,7 @@ int cg_create(int n, int C, int K, const uint32_t* c0, const uint32_t* c1, const
         chk(cudaMalloc(&s->kspec, sizeof(float2) * K * (half + n)), "cudaMalloc(kspec)");
         chk(cudaMalloc(&s->kspec_re, sizeof(float) * K * (half + n)), "cudaMalloc(kspec_re)");
         s->kreal.assign(size_t(K), 0);
+    s->kset.assign(size_t(K), 0);
     if (rc == CG_OK) chk(cudaMalloc(&s->U, 2 * sizeof(float2) * K * half), "cudaMalloc(U)");
     if (rc == CG_OK) chk(cudaMalloc(&s->A, sizeof(float) * C * px), "cudaMalloc(A)");
     if (rc == CG_OK)
@@ -661,7 +698,6 @@ int cg_create(int n, int C, int K, const uint32_t* c0, const uint32_t* c1, const
     if (rc == CG_OK)
         chk(cudaMemsetAsync(s->kspec, 0, sizeof(float2) * K * (half + n), s->stream), "memset");
     if (rc == CG_OK) rc = build_twiddles(s);
-    if (rc == CG_OK) rc = capture_graphs(s);
     if (rc == CG_OK) chk(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
     if (rc != CG_OK) {
         release(s);
@@ -684,16 +720,25 @@ int cg_destroy(cg_sim* s) {
 namespace {
 // Record whether kernel k's spectrum is real (k < 0: every kernel not real);
 // when the world's column pass changes between the real and the complex
-// form, re-capture the step graphs.
+// form, re-capture the step graphs; with the last kernel's first upload,
+// capture them.
 int set_kernel_realness(cg_sim* s, int k, bool real) {
     if (k >= 0) s->kreal[size_t(k)] = real ? 1 : 0;
     else std::fill(s->kreal.begin(), s->kreal.end(), uint8_t(0));
     bool all = true;
     for (uint8_t r : s->kreal) all = all && r != 0;
-    if (all == s->kreal_all) return CG_OK;
-    CG_CHECK(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
-    s->kreal_all = all;
-    return recapture(s);
+    bool complete = false;
+    if (k >= 0 && !s->graphs_ready) {
+        s->kset[size_t(k)] = 1;
+        complete = true;
+        for (uint8_t u : s->kset) complete = complete && u != 0;
+    }
+    if (all == s->kreal_all && !complete) return CG_OK;
+    if (all != s->kreal_all) {
+        CG_CHECK(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
+        s->kreal_all = all;
+    }
+    return complete ? capture_graphs(s) : recapture(s);
 }
 }  // namespace
 
@@ -759,15 +804,21 @@ int cg_upload_channel_f32(cg_sim* s, int c, const float* data) {
 int cg_step(cg_sim* s, int nsteps) {
     if (!s) return fail(CG_ERR_ARG, "cg_step: NULL handle");
     if (nsteps < 0) return fail(CG_ERR_ARG, "negative step count %d", nsteps);
-    int left = nsteps;
-    while (left >= kStepsPerGraph) {   // an even count: the parity is unchanged
-        CG_CHECK(cudaGraphLaunch(s->graph8[s->cur], s->stream), "cudaGraphLaunch");
-        left -= kStepsPerGraph;
+    bool direct = false;
+    if (nsteps > 0) {
+        const int rc = ensure_graphs(s, s->stream, &direct);
+        if (rc != CG_OK) return rc;
     }
-    for (; left > 0; --left) {
-        CG_CHECK(cudaGraphLaunch(s->graph[s->cur], s->stream), "cudaGraphLaunch");
-        s->cur ^= 1;
+    for (int i = 0; direct && i < nsteps; ++i) {
+        const int rc = step_direct(s, s->stream, false);
+        if (rc != CG_OK) return rc;
     }
+    int left = direct ? 0 : nsteps;
+    for (int i = 0; i < 4; ++i)
+        for (; left >= kGraphSteps[i]; left -= kGraphSteps[i]) {
+            CG_CHECK(cudaGraphLaunch(s->graph[i][s->cur], s->stream), "cudaGraphLaunch");
+            s->cur ^= kGraphSteps[i] & 1;
+        }
     return CG_OK;
 }
 
@@ -775,6 +826,10 @@ int cg_iterate(cg_sim* s) { return cg_step(s, 1); }
 
 int cg_iterate_and_render(cg_sim* s) {
     if (!s) return fail(CG_ERR_ARG, "cg_iterate_and_render: NULL handle");
+    bool direct = false;
+    const int rc = ensure_graphs(s, s->stream, &direct);
+    if (rc != CG_OK) return rc;
+    if (direct) return step_direct(s, s->stream, true);
     CG_CHECK(cudaGraphLaunch(s->graphR[s->cur], s->stream), "cudaGraphLaunch");
     s->cur ^= 1;
     return CG_OK;
@@ -874,7 +929,11 @@ int cg_render_ptr(cg_sim* s, const uint32_t** out) {
 int cg_iterate_on(cg_sim* s, cg_stream_t stream) {
     if (!s) return fail(CG_ERR_ARG, "cg_iterate_on: NULL handle");
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : s->stream;
-    CG_CHECK(cudaGraphLaunch(s->graph[s->cur], st), "cudaGraphLaunch");
+    bool direct = false;
+    const int rc = ensure_graphs(s, st, &direct);
+    if (rc != CG_OK) return rc;
+    if (direct) return step_direct(s, st, false);
+    CG_CHECK(cudaGraphLaunch(s->graph[kOneStep][s->cur], st), "cudaGraphLaunch");
     s->cur ^= 1;
     return CG_OK;
 }
