@@ -177,16 +177,19 @@ class _UnrollRings(torch.autograd.Function):
         gtmp = torch.empty_like(gT)
         seg = torch.empty((ctx.every,) + tuple(gT.shape), dtype=torch.float32, device=gT.device)
         K, n = world.K, world.n
-        pgrad = torch.zeros(3 * K, dtype=torch.float64, device=gT.device)
-        kgrad = torch.zeros((K, n // 2, n, 2), dtype=torch.float32, device=gT.device)
+        pgrad = torch.empty(3 * K, dtype=torch.float64, device=gT.device)
+        kgrad = torch.empty((K, n // 2, n, 2), dtype=torch.float32, device=gT.device)
+        check(lib.cg_zero_grads(world.h, _p(pgrad), _p(kgrad)))
         check(lib.cg_unroll_backward(world.h, _p(ckpt), ctx.T, ctx.every, _p(gT), _p(g0),
                                      _p(pgrad), _p(kgrad), _p(seg), _p(gtmp)))
         hbar = torch.empty((K, n, n), dtype=torch.float32, device=gT.device)
         check(lib.cg_kernel_grad_spatial(world.h, _p(kgrad), _p(hbar)))
-        grings = torch.zeros_like(rw)
+        grings = torch.empty_like(rw)   # every entry is written
         check(lib.cg_ring_weight_grad(world.h, ctypes.cast(ctx.specs, ctypes.c_void_p), _p(rw),
                                       _p(hbar), _p(grings)))
         ds, dm, dsg, dw, dr = ctx.dtypes
+        if dm == dsg == dw:   # one conversion for the three
+            pgrad = pgrad.to(dm)
         return (None, None, None, None, g0.to(ds), pgrad[:K].to(dm), pgrad[K:2 * K].to(dsg),
                 pgrad[2 * K:].to(dw), grings.to(dr))
 
@@ -245,6 +248,7 @@ class DiffusionLeniaGPU(torch.nn.Module):
                                          device=device)
         from .orchestrator import creature_ring_specs, ring_spec_array
         self.specs = ring_spec_array(creature_ring_specs(cr)[0])
+        self._ring_counts, self._ring_slots = None, None   # rings()
 
     def kernels(self):
         """The spatial kernels (K, n, n) as differentiable torch ops (float64)."""
@@ -252,8 +256,18 @@ class DiffusionLeniaGPU(torch.nn.Module):
 
     def rings(self):
         """Ring weights padded to (K, 8), differentiable."""
-        return torch.stack([torch.nn.functional.pad(b, (0, _abi.MAX_RINGS - b.numel()))
-                            for b in self.ring_weights])
+        # one concatenation and one scatter: a pad per kernel, the stack and
+        # their backward were a fifth of a small creature's host time
+        weights = list(self.ring_weights)
+        counts = tuple(b.numel() for b in weights)
+        if counts != self._ring_counts:
+            self._ring_counts = counts
+            self._ring_slots = torch.tensor(
+                [k * _abi.MAX_RINGS + l for k, c in enumerate(counts) for l in range(c)],
+                device=self.world.device)
+        flat = torch.cat(weights)
+        padded = flat.new_zeros(len(weights) * _abi.MAX_RINGS)
+        return padded.index_copy(0, self._ring_slots, flat).view(-1, _abi.MAX_RINGS)
 
     def forward(self, T: int, every: int = 8):
         """x_T; the kernels are built on the GPU from the ring weights."""
