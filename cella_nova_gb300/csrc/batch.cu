@@ -468,9 +468,12 @@ cudaError_t enqueue_class_steps(cg_batch* b, const cg_batch::SizeClass& sc, int 
         cudaEvent_t* ec2r = ecol + W.C;
         ev += 2 * size_t(W.C);
         for (int t = 0; t < nsteps && e == cudaSuccess; ++t) {
-            const StepArgs a = world_step_args(b, w, parity_at(t), var);
+            StepArgs a = world_step_args(b, w, parity_at(t), var);
+            // a small world's diffusion takes the next step's row pass with it
+            const bool fuse = fuses_next_row(sc.logn, var);
+            if (fuse && t + 1 < nsteps) a.rowspec_next = W.rowspec;
             for (int c = 0; c < W.C && e == cudaSuccess; ++c) {
-                e = ops->step_channel(a, kPhaseRowFwd, c, ls[c]);
+                if (t == 0 || !fuse) e = ops->step_channel(a, kPhaseRowFwd, c, ls[c]);
                 // a column pass overwrites U, which every channel's inverse
                 // row pass of the step before read
                 for (int o = 0; t > 0 && o < W.C && e == cudaSuccess; ++o)

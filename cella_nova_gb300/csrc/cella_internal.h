@@ -77,10 +77,19 @@ struct StepArgs {
     float* udbg;   // optional [K][n][n] f32: Re(conv) before the 1/n^2 scale
     int* err;      // device error word (bounded waits that timed out)
     unsigned char* levels;   // optional [3][n][n] render level bytes, written by the diffusion
+    // optional (fuses_next_row): the diffusion kernel also transforms the rows
+    // of x_out into these row spectra, the next step's kPhaseRowFwd
+    float2* rowspec_next;
     KernelGroups groups;
     const GrowthParams* gp;   // device-resident: updated without re-capturing graphs
     Variants var;
 };
+
+// Whether a world's diffusion can take the next step's forward row pass with
+// it: small sides, and a forward row pass of variants 0-2, whose bits it gives.
+inline bool fuses_next_row(int logn, const Variants& var) {
+    return logn <= kMaxSmallLogN && var.r2c <= 2;
+}
 
 // Per-kernel constants of the backward pass.
 struct AdjointParams {

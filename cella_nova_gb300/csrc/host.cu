@@ -346,6 +346,17 @@ constexpr int kGraphSteps[4] = {8, 4, 2, 1};
 constexpr int kStepsPerGraph = kGraphSteps[0];
 constexpr int kOneStep = 3;   // index of the one-step graph
 
+// Phases of a step in a chain of steps: where the world's diffusion takes the
+// next step's forward row pass with it (into a->rowspec_next, by default the
+// world's own row spectra), a step after another has that phase behind it, and
+// one before another asks for it.
+int chain_step(const cg_sim* s, StepArgs* a, bool after, bool before,
+               float2* rowspec_next = nullptr) {
+    if (!fuses_next_row(s->logn, s->var)) return kPhaseAll;
+    if (before) a->rowspec_next = rowspec_next ? rowspec_next : s->rowspec;
+    return after ? kPhaseAll & ~kPhaseRowFwd : int(kPhaseAll);
+}
+
 // Capture `nsteps` steps starting at ping-pong parity p0 as one graph whose
 // launches are per channel, on one stream per channel, so that independent
 // channels overlap (one channel's diffusion runs in another's tail).  Only
@@ -382,7 +393,7 @@ cudaError_t capture_steps(cg_sim* s, int p0, int nsteps, bool render, cudaGraphE
                     a.x_out = s->state[p0 ^ 1];
                 }
                 if (render && t == nsteps - 1) a.levels = s->levels;
-                le = s->ops->step(a, kPhaseAll, st0);
+                le = s->ops->step(a, chain_step(s, &a, t > 0, t + 1 < nsteps), st0);
             }
             if (render && le == cudaSuccess)
                 le = launch_pack_levels(s->levels, C, s->px(), s->render, st0);
@@ -418,8 +429,9 @@ cudaError_t capture_steps(cg_sim* s, int p0, int nsteps, bool render, cudaGraphE
                 a.x_out = s->state[p0 ^ 1];
             }
             if (render && t == nsteps - 1) a.levels = s->levels;
+            const int phases = chain_step(s, &a, t > 0, t + 1 < nsteps);
             for (int c = 0; c < C && le == cudaSuccess; ++c) {
-                le = s->ops->step_channel(a, kPhaseRowFwd, c, st[c]);
+                if (phases & kPhaseRowFwd) le = s->ops->step_channel(a, kPhaseRowFwd, c, st[c]);
                 // U alternates with the parity, so the column pass of step t
                 // only has to wait for the inverse row passes of step t-2,
                 // which read the same buffer
@@ -1304,8 +1316,12 @@ int cg_unroll(cg_sim* s, const float* x0, int T, int every, float* ckpt, float* 
         if (t + 1 == T) nxt = xT;
         else if ((t + 1) % every == 0) nxt = ckpt + plane * size_t((t + 1) / every);
         else nxt = s->utmp[(t + 1) & 1];
-        int rc = cg_step_from(s, cur, nxt);
-        if (rc != CG_OK) return rc;
+        if (cur == nxt) return fail(CG_ERR_ARG, "cg_unroll: a step's input and output must differ");
+        StepArgs a = s->args(s->cur, nullptr);
+        a.x_in = cur;
+        a.x_out = nxt;
+        CG_CHECK(s->ops->step(a, chain_step(s, &a, t > 0, t + 1 < T), s->stream),
+                 "launching a step");
         cur = nxt;
     }
     return CG_OK;
@@ -1361,8 +1377,15 @@ int cg_unroll_backward(cg_sim* s, const float* ckpt, int T, int every, const flo
             a.x_in = seg + plane * size_t(t - t0);
             const bool last = t + 1 == t1;
             a.x_out = last ? nullptr : seg + plane * size_t(t - t0 + 1);
-            CG_CHECK(s->ops->step(a, last ? (kPhaseRowFwd | kPhaseColConv | kPhaseGrowth) : kPhaseAll,
-                                  s->stream),
+            float2* next_rows = nullptr;
+            if (!last) {
+                float2* next_U;
+                float* next_A;
+                slot(t - t0 + 1, &next_rows, &next_U, &next_A);
+            }
+            int phases = chain_step(s, &a, t > t0, !last, next_rows);
+            if (last) phases &= ~kPhaseDiffusion;
+            CG_CHECK(s->ops->step(a, phases, s->stream),
                      "recomputing a segment");
         }
         for (int t = t1 - 1; t >= t0; --t) {

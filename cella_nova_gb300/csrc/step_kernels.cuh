@@ -1225,6 +1225,128 @@ __global__ void __launch_bounds__(DiffTile<LOGN, V>::THREADS)
 }
 
 // ---------------------------------------------------------------------------
+// Diffusion and the next step's forward row pass in one kernel (small sides):
+// a CTA takes RB whole rows, so the new rows are in shared memory when their
+// transform begins.  It saves a launch of the four of a step and the reload of
+// the state; at these sides a launch is 2 to 3 us whatever it does.  The rows
+// above and below a CTA's are read twice, which at 2048^2 would cost what it
+// saves (q for 1.5 rows per row).  Same arithmetic, order and plan as
+// diffusion2_body and row_r2c_body, so the same bits as the two kernels.
+// grid (N/RB, C), block T.
+// ---------------------------------------------------------------------------
+template <int LOGN>
+struct DiffRowGeo : Geo<LOGN, 0> {
+    using G = Geo<LOGN, 0>;
+    static constexpr int N = G::N, RB = G::RB;
+    // a thread owns a column (two at 512) of all the rows, or of half of them
+    static constexpr int RT = N < 128 ? 2 * N : (N < 256 ? N : 256);
+    static constexpr int SEG = RT > N ? 2 : 1, CPT = RT > N ? 1 : N / RT;
+    static constexpr int AH = RB + 4, QH = RB + 2;   // rows of A and of q
+    static constexpr int V4 = N / 4;                 // 16-byte loads per A row
+    static constexpr int LOADS = (AH * V4 + RT - 1) / RT;
+    static constexpr int ROWS = (2 * AH + QH) * N;   // floats before the work rows
+    static constexpr size_t SMEM = ROWS * sizeof(float) + G::R2C_SMEM;
+    static_assert(QH % SEG == 0 && RB % SEG == 0 && ROWS % 4 == 0, "row segments");
+};
+
+template <int LOGN>
+__global__ void __launch_bounds__(DiffRowGeo<LOGN>::RT)
+    k_diff_r2c(const float* __restrict__ A, const float* __restrict__ x, float* __restrict__ out,
+               float2* __restrict__ rowspec, const float2* __restrict__ tw, int cbase) {
+    using D = DiffRowGeo<LOGN>;
+    constexpr int N = D::N, T = D::RT, MASK = N * N - 1;
+    extern __shared__ __align__(128) float sm_dr[];
+    float* sAh = sm_dr;               // [AH][N]: row a <-> y0 + a - 2, heads
+    float* sAl = sAh + D::AH * N;     // tails
+    float* sQ = sAl + D::AH * N;      // [QH][N]: row b <-> y0 + b - 1
+    float2* rows = reinterpret_cast<float2*>(sm_dr + D::ROWS);   // the new rows, as pairs
+    warm_table<T>(tw + D::TW_ROW, tw_size(D::M, false));
+    warm_table<T>(tw, D::M / 2);
+    pdl_wait();
+    pdl_launch_dependents();
+    const int c = blockIdx.y + cbase, y0 = blockIdx.x * D::RB, t = threadIdx.x;
+    const float* Ac = A + size_t(c) * N * N;
+    const float* xc = x + size_t(c) * N * N;
+    constexpr int ZR = D::QH / D::SEG, OR = D::RB / D::SEG;
+    const int seg = t / N, col0 = t % N;   // seg 0 where a thread takes whole columns
+
+    float xv[D::CPT][ZR];
+#pragma unroll
+    for (int i = 0; i < D::CPT; ++i)
+#pragma unroll
+        for (int b = 0; b < ZR; ++b)
+            xv[i][b] = __ldg(xc + (((y0 + seg * ZR + b - 1) * N) & MASK) + col0 + i * T);
+    float4 av[D::LOADS];
+#pragma unroll
+    for (int i = 0; i < D::LOADS; ++i) {
+        const int e = t + i * T;
+        if (D::AH * D::V4 % T == 0 || e < D::AH * D::V4)
+            av[i] = __ldg(reinterpret_cast<const float4*>(
+                Ac + (((y0 + e / D::V4 - 2) * N) & MASK) + 4 * (e % D::V4)));
+    }
+#pragma unroll
+    for (int i = 0; i < D::LOADS; ++i) {
+        const int e = t + i * T;
+        if (D::AH * D::V4 % T == 0 || e < D::AH * D::V4) {
+            const float4 a = av[i];
+            const float4 h = make_float4(head12(a.x), head12(a.y), head12(a.z), head12(a.w));
+            *reinterpret_cast<float4*>(sAh + 4 * e) = h;
+            *reinterpret_cast<float4*>(sAl + 4 * e) =
+                make_float4(a.x - h.x, a.y - h.y, a.z - h.z, a.w - h.w);
+        }
+    }
+    __syncthreads();
+    // the horizontal 3-sum around a column, toroidal
+    auto sum3 = [](const float* p, int l, int m, int r) { return p[l] + p[m] + p[r]; };
+#pragma unroll
+    for (int i = 0; i < D::CPT; ++i) {
+        const int m = col0 + i * T, l = (m - 1) & (N - 1), r = (m + 1) & (N - 1);
+        const float* ph = sAh + seg * ZR * N;
+        const float* pl = sAl + seg * ZR * N;
+        float h0 = sum3(ph, l, m, r), l0 = sum3(pl, l, m, r);
+        float h1 = sum3(ph + N, l, m, r), l1 = sum3(pl + N, l, m, r);
+#pragma unroll
+        for (int b = 0; b < ZR; ++b) {
+            const float h2 = sum3(ph + (b + 2) * N, l, m, r);
+            const float l2 = sum3(pl + (b + 2) * N, l, m, r);
+            const float zh = h0 + h1 + h2;
+            const float zt = l0 + l1 + l2;
+            sQ[(seg * ZR + b) * N + m] = div_head_tail(xv[i][b], zh, zt);
+            h0 = h1;
+            l0 = l1;
+            h1 = h2;
+            l1 = l2;
+        }
+    }
+    __syncthreads();
+    float* oc = out + (size_t(c) * N + y0 + seg * OR) * N;
+    float* zr = reinterpret_cast<float*>(rows + seg * OR * D::RP);
+#pragma unroll
+    for (int i = 0; i < D::CPT; ++i) {
+        const int m = col0 + i * T, l = (m - 1) & (N - 1), r = (m + 1) & (N - 1);
+        const float* pq = sQ + seg * OR * N;
+        const float* pa = sAh + (seg * OR + 2) * N + m;
+        const float* pb = sAl + (seg * OR + 2) * N + m;
+        float s0 = sum3(pq, l, m, r), s1 = sum3(pq + N, l, m, r);
+#pragma unroll
+        for (int b = 0; b < OR; ++b) {
+            const float s2 = sum3(pq + (b + 2) * N, l, m, r);
+            const float a = pa[b * N] + pb[b * N];
+            const float v = a * ((s0 + s1) + s2);
+            oc[b * N + m] = v;
+            zr[2 * (b * D::RP + pidx(m >> 1)) + (m & 1)] = v;
+            s0 = s1;
+            s1 = s2;
+        }
+    }
+    __syncthreads();
+    SmemRows work{rows, D::RP};
+    FftPasses<D::M, 1, false, T, D::RB, false, D::ROW_MR>::run(work, work, work, work,
+                                                             tw + D::TW_ROW);
+    r2c_finish<D>(rows, tw, rowspec + size_t(c) * D::M * N + y0);
+}
+
+// ---------------------------------------------------------------------------
 // Kernel spectrum packing (set_kernel, mod.rs:207-214): full n x n spectrum
 // [ky][kx] -> Hermitian part, scaled by 1/(2 n^2), kx-major [kx][ky] for
 // kx in [1, n/2), with the alpha/beta pair in columns 0 and n/2.
@@ -1296,6 +1418,11 @@ cudaError_t prepare_size() {
         if (e == cudaSuccess) e = prepare_variant<LOGN, 4>();
     }
     if (e == cudaSuccess) e = prepare_c2r_debug<LOGN>();
+    if constexpr (LOGN <= kMaxSmallLogN) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_diff_r2c<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(DiffRowGeo<LOGN>::SMEM));
+    }
     if (e == cudaSuccess) e = prepare_diffusion<LOGN, 0>();
     if (e == cudaSuccess) e = prepare_diffusion<LOGN, 1>();
     if (e == cudaSuccess) e = prepare_diffusion<LOGN, 2>();
@@ -1443,7 +1570,16 @@ cudaError_t launch_step_range(const StepArgs& a, int phases, int c_lo, int c_hi,
     if (phases & kPhaseGrowth) { CG_VARIANT_SWITCH5(a.var.c2r, e = launch_c2r, a, c_lo, nc, st) }
     if (e != cudaSuccess) return e;
     if (phases & kPhaseDiffusion) {
-        CG_DIFF_SWITCH(a.var.diff, e = launch_diff, a, c_lo, nc, st)
+        bool fused = false;
+        if constexpr (LOGN <= kMaxSmallLogN) {
+            if (a.rowspec_next) {
+                using D = DiffRowGeo<LOGN>;
+                fused = true;
+                e = launch_pdl(k_diff_r2c<LOGN>, dim3(D::N / D::RB, nc), D::RT, D::SMEM, st, a.A,
+                               a.x_in, a.x_out, a.rowspec_next, a.tw, c_lo);
+            }
+        }
+        if (!fused) { CG_DIFF_SWITCH(a.var.diff, e = launch_diff, a, c_lo, nc, st) }
     }
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
