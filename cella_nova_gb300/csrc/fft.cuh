@@ -185,6 +185,22 @@ __host__ __device__ constexpr int plan_last_radix(int L, bool remfirst, int MR =
 //   twp : this pass's table (tw_offset layout).
 //   ld(s, i, it, q)         -> float2
 //   st(s, i, v, it, q)      (it, q) name the register slot of the value.
+// The threads that share a transform: the whole CTA, or groups of GT
+// consecutive threads that each run a transform of their own (barrier g + 1
+// for group g, or the warp's own where a group is one).
+struct CtaThreads {
+    __device__ __forceinline__ static int tid() { return threadIdx.x; }
+    __device__ __forceinline__ static void sync() { __syncthreads(); }
+};
+template <int GT>
+struct GroupThreads {
+    __device__ __forceinline__ static int tid() { return threadIdx.x % GT; }
+    __device__ __forceinline__ static void sync() {
+        if constexpr (GT == 32) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(threadIdx.x / GT + 1), "n"(GT) : "memory");
+    }
+};
+
 template <int S, int J, bool SFAST>
 __device__ __forceinline__ void item_pos(int item, int& s, int& j) {
     if constexpr (SFAST) {
@@ -197,7 +213,7 @@ __device__ __forceinline__ void item_pos(int item, int& s, int& j) {
 }
 
 template <int L, int R, int NS, bool INV, int T, int S, bool SFAST = false, bool MIDBAR = true,
-          class LD, class ST>
+          class PAR = CtaThreads, class LD, class ST>
 __device__ __forceinline__ void stockham_pass(LD& ld, ST& st, const float2* __restrict__ twp) {
     constexpr int J = L / R;
     constexpr int ITEMS = S * J;
@@ -205,7 +221,7 @@ __device__ __forceinline__ void stockham_pass(LD& ld, ST& st, const float2* __re
     float2 v[IPT][R];
 #pragma unroll
     for (int it = 0; it < IPT; ++it) {
-        const int item = threadIdx.x + it * T;
+        const int item = PAR::tid() + it * T;
         if (ITEMS % T == 0 || item < ITEMS) {
             int s, j;
             item_pos<S, J, SFAST>(item, s, j);
@@ -219,10 +235,10 @@ __device__ __forceinline__ void stockham_pass(LD& ld, ST& st, const float2* __re
             }
         }
     }
-    if constexpr (MIDBAR) __syncthreads();
+    if constexpr (MIDBAR) PAR::sync();
 #pragma unroll
     for (int it = 0; it < IPT; ++it) {
-        const int item = threadIdx.x + it * T;
+        const int item = PAR::tid() + it * T;
         if (ITEMS % T == 0 || item < ITEMS) {
             int s, j;
             item_pos<S, J, SFAST>(item, s, j);
@@ -247,7 +263,7 @@ __device__ __forceinline__ void stockham_pass(LD& ld, ST& st, const float2* __re
             }
         }
     }
-    __syncthreads();
+    PAR::sync();
 }
 
 // Full length-L transform: first pass reads through `ld`, middle passes use
@@ -258,7 +274,7 @@ __device__ __forceinline__ void stockham_pass(LD& ld, ST& st, const float2* __re
 // MIDBAR): for a first pass whose `ld` reads no shared memory that smst
 // writes, and a last pass whose `stl` writes no shared memory smld reads.
 template <int L, int NS, bool INV, int T, int S, bool REMFIRST = false, int MR = 16,
-          bool SFAST = false, bool FIRSTBAR = true, bool LASTBAR = true>
+          bool SFAST = false, bool FIRSTBAR = true, bool LASTBAR = true, class PAR = CtaThreads>
 struct FftPasses {
     template <class LD, class SMLD, class SMST, class STL>
     __device__ __forceinline__ static void run(LD& ld, SMLD& smld, SMST& smst, STL& stl,
@@ -269,10 +285,10 @@ struct FftPasses {
                                            : (FIRST ? FIRSTBAR : (LAST ? LASTBAR : true));
         const float2* twp = tab + tw_offset(L, REMFIRST, NS, MR);
         if constexpr (LAST) {
-            stockham_pass<L, R, NS, INV, T, S, SFAST, BAR>(ld, stl, twp);
+            stockham_pass<L, R, NS, INV, T, S, SFAST, BAR, PAR>(ld, stl, twp);
         } else {
-            stockham_pass<L, R, NS, INV, T, S, SFAST, BAR>(ld, smst, twp);
-            FftPasses<L, NS * R, INV, T, S, REMFIRST, MR, SFAST, FIRSTBAR, LASTBAR>::run(
+            stockham_pass<L, R, NS, INV, T, S, SFAST, BAR, PAR>(ld, smst, twp);
+            FftPasses<L, NS * R, INV, T, S, REMFIRST, MR, SFAST, FIRSTBAR, LASTBAR, PAR>::run(
                 smld, smld, smst, stl, tab);
         }
     }
@@ -281,19 +297,19 @@ struct FftPasses {
 // Run the first pass of a transform, then `hook()`, then the rest.
 // FIRSTBAR / LASTBAR as in FftPasses.
 template <int L, bool INV, int T, int S, bool REMFIRST, int MR = 16, bool SFAST = false,
-          bool FIRSTBAR = true, bool LASTBAR = true, class LD, class SMLD, class SMST, class STL,
-          class HOOK>
+          bool FIRSTBAR = true, bool LASTBAR = true, class PAR = CtaThreads, class LD, class SMLD,
+          class SMST, class STL, class HOOK>
 __device__ __forceinline__ void fft_with_hook(LD& ld, SMLD& smld, SMST& smst, STL& stl,
                                               const float2* __restrict__ tab, HOOK hook) {
     constexpr int R = PassRadix<L, 1, REMFIRST, MR>::R;
     if constexpr (R == L) {
-        stockham_pass<L, R, 1, INV, T, S, SFAST, FIRSTBAR || LASTBAR>(ld, stl, tab);
+        stockham_pass<L, R, 1, INV, T, S, SFAST, FIRSTBAR || LASTBAR, PAR>(ld, stl, tab);
         hook();
     } else {
-        stockham_pass<L, R, 1, INV, T, S, SFAST, FIRSTBAR>(ld, smst, tab);
+        stockham_pass<L, R, 1, INV, T, S, SFAST, FIRSTBAR, PAR>(ld, smst, tab);
         hook();
-        FftPasses<L, R, INV, T, S, REMFIRST, MR, SFAST, true, LASTBAR>::run(smld, smld, smst, stl,
-                                                                             tab);
+        FftPasses<L, R, INV, T, S, REMFIRST, MR, SFAST, true, LASTBAR, PAR>::run(smld, smld, smst,
+                                                                                 stl, tab);
     }
 }
 

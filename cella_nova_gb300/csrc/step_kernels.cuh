@@ -765,6 +765,140 @@ __global__ void __launch_bounds__(C2RShape<LOGN, V>::RT, C2RShape<LOGN, V>::MINB
 }
 
 // ---------------------------------------------------------------------------
+// The same at small sides with the kernels of the channel side by side: group
+// g of GT threads transforms kernel g, then g + the number of groups, ...,
+// and leaves the bump's values e in shared memory; the whole CTA then adds
+// w e in increasing k (the order and the bits of row_c2r_growth_body) and
+// writes A.  One CTA of 32 or 64 threads with three kernels one after another
+// is a chain of three transforms on an SM that has nothing else to do:
+// 4.4 -> 3.7 us at 256^2 with C=3, K=9.  At 512^2
+// the CTAs of row_c2r_growth_body already fill the GPU and win (5.7 against
+// 6.1 us).
+// grid (N/RB, C), block GT * groups.
+// ---------------------------------------------------------------------------
+constexpr int kMaxGroups = 4, kMaxGroupsLogN = 8;
+template <int LOGN>
+struct C2RGroups : Geo<LOGN, 0> {
+    using G = Geo<LOGN, 0>;
+    static constexpr int GT = G::RT;
+    static constexpr int PITCH = G::C2R_LAND + G::C2R_TILE;   // float2 per group
+    static constexpr size_t SMEM = size_t(PITCH) * sizeof(float2);
+    static_assert(SMEM % 128 == 0, "tensor-copy destination alignment");
+};
+
+template <int LOGN>
+__global__ void __launch_bounds__(C2RGroups<LOGN>::GT* kMaxGroups)
+    k_row_c2r_groups(const __grid_constant__ CUtensorMap umap, float* __restrict__ A,
+                     const float2* __restrict__ tw, const __grid_constant__ KernelGroups groups,
+                     const GrowthParams* __restrict__ gpp, float temp, int* err, int cbase) {
+    using G = C2RGroups<LOGN>;
+    using PAR = GroupThreads<G::GT>;
+    constexpr int N = G::N, M = G::M, RB = G::RB, GT = G::GT;
+    constexpr int RL = last_radix(M, G::ROW_MR), JL = M / RL, ITEMS = RB * JL;
+    constexpr int SLOTS = RB * M;   // pixel pairs of the CTA's rows
+    constexpr int SPT = (SLOTS + 2 * GT - 1) / (2 * GT);   // per thread, with two groups or more
+    constexpr uint32_t kTileBytes = uint32_t(G::C2R_TILE) * sizeof(float2);
+    extern __shared__ __align__(128) float2 sm_c2rg[];
+    __shared__ __align__(8) uint64_t bars[kMaxGroups];
+    const int g = threadIdx.x / GT, ng = blockDim.x / GT, tid = threadIdx.x % GT;
+    const int c = blockIdx.y + cbase, y0 = blockIdx.x * RB;
+    const int cnt = groups.out_count[c], base = groups.out_start[c];
+    float2* work = sm_c2rg + g * G::PITCH;   // this group's rows, then the bump's values
+    float2* land = work + G::C2R_LAND;
+    uint64_t* bar = bars + g;
+    init_tile_barriers<kMaxGroups>(bars);
+    warm_table<GT>(tw + G::TW_ROW, tw_size(M, false));
+    warm_table<GT>(tw, M);   // W_N^m of the pre-split
+    pdl_wait();
+    pdl_launch_dependents();
+    auto issue = [&](int gi) {   // the group's first thread copies
+        if (tid != 0) return;
+        const int k = groups.out_idx[base + gi];
+        mbar_arrive_expect_tx(bar, kTileBytes);
+#pragma unroll
+        for (int q = 0; q < M / G::UBOX; ++q)
+            tensor2d_g2s(land + q * G::UBOX * RB, &umap, 2 * y0, k * M + q * G::UBOX, bar);
+    };
+    if (g < cnt) issue(g);
+    float2 acc[SPT];
+#pragma unroll
+    for (int i = 0; i < SPT; ++i) acc[i] = make_float2(0.f, 0.f);
+    const GrowthParams& gp = *gpp;
+    uint32_t phase = 0;
+    for (int first = 0; first < cnt; first += ng) {
+        const int gi = first + g;
+        bool ok = true;
+        if (gi < cnt) {
+            // a wait that timed out computes on what is there; the CTA leaves
+            // at the barrier below
+            ok = mbar_wait(bar, phase & 1u, err);
+            ++phase;
+            const float2* lt = land + tid % RB;   // lt[kx * RB]
+            auto ld0 = [&](int, int m, int, int q) -> float2 {
+                if (q == 0 && m == 0) {
+                    const float2 x = lt[0];
+                    return make_float2(x.x + x.y, x.x - x.y);
+                }
+                const float2 a = lt[m * RB];
+                const float2 b = cconj(lt[(M - m) * RB]);
+                const float2 E = cadd(a, b);
+                const float2 O = cmulc(csub(a, b), __ldg(&tw[m]));
+                return make_float2(E.x - O.y, E.y + O.x);
+            };
+            const int k = groups.out_idx[base + gi];
+            const float mu = gp.mu[k], c2 = gp.c2[k];
+            auto bump = [&](int, int, float2 v, int it, int r) {
+                const float dx = v.x - mu, dy = v.y - mu;
+                work[r * ITEMS + tid + it * GT] =
+                    make_float2(ex2_approx(dx * dx * c2), ex2_approx(dy * dy * c2));
+            };
+            SmemRows rows{work, G::RP};
+            fft_with_hook<M, true, GT, RB, false, G::ROW_MR, true, false, true, PAR>(
+                ld0, rows, rows, bump, tw + G::TW_ROW, [&]() {
+                    if (gi + ng < cnt) {   // the first pass has read the tile
+                        fence_proxy_async_smem();
+                        PAR::sync();
+                        issue(gi + ng);
+                    }
+                });
+        }
+        if (__syncthreads_or(!ok)) {
+            // the copies in flight get one more bounded chance to land before
+            // this CTA's shared memory is released
+            if (gi < cnt) mbar_wait(bar, (phase - 1) & 1u, nullptr);
+            if (gi + ng < cnt) mbar_wait(bar, phase & 1u, nullptr);
+            return;
+        }
+        for (int q = 0; q < ng && first + q < cnt; ++q) {
+            const float w2 = gp.w2[groups.out_idx[base + first + q]];
+            const float2* e = sm_c2rg + q * G::PITCH;
+#pragma unroll
+            for (int i = 0; i < SPT; ++i) {
+                const int slot = threadIdx.x + i * blockDim.x;
+                if (slot < SLOTS) {
+                    acc[i].x = fmaf(w2, e[slot].x, acc[i].x);
+                    acc[i].y = fmaf(w2, e[slot].y, acc[i].y);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    float* Ac = A + (size_t(c) * N + y0) * N;
+    const float tl = temp * 1.44269504088896341f;   // temp log2(e)
+    const float toff = -tl * gp.wsum[c];
+#pragma unroll
+    for (int i = 0; i < SPT; ++i) {
+        const int slot = threadIdx.x + i * blockDim.x;
+        if (slot < SLOTS) {
+            int s, j;
+            item_pos<RB, JL, true>(slot % ITEMS, s, j);
+            reinterpret_cast<float2*>(Ac + size_t(s) * N)[j + slot / ITEMS * JL] = make_float2(
+                ex2_approx(fmaf(tl, acc[i].x, toff)), ex2_approx(fmaf(tl, acc[i].y, toff)));
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Diffusion: Z = toroidal 3x3 sum of A, new = A * (3x3 sum of state / Z)
 // (example.rs:272-303, compute_1024.wgsl:341-413).  One channel tile per
 // CTA; A is read with a 2-pixel halo and the state with a 1-pixel halo, so
@@ -1423,6 +1557,12 @@ cudaError_t prepare_size() {
             e = cudaFuncSetAttribute(k_diff_r2c<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      int(DiffRowGeo<LOGN>::SMEM));
     }
+    if constexpr (LOGN <= kMaxGroupsLogN) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_row_c2r_groups<LOGN>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(kMaxGroups * C2RGroups<LOGN>::SMEM));
+    }
     if (e == cudaSuccess) e = prepare_diffusion<LOGN, 0>();
     if (e == cudaSuccess) e = prepare_diffusion<LOGN, 1>();
     if (e == cudaSuccess) e = prepare_diffusion<LOGN, 2>();
@@ -1507,6 +1647,21 @@ cudaError_t launch_c2r_shape(const StepArgs& a, int c_lo, int nc, cudaStream_t s
 template <int LOGN, int V>
 cudaError_t launch_c2r(const StepArgs& a, int c_lo, int nc, cudaStream_t st) {
     if (a.udbg) return launch_c2r_shape<LOGN, 0, true>(a, c_lo, nc, st);
+    if constexpr (V == 0 && LOGN <= kMaxGroupsLogN) {
+        int most = 1;
+        for (int c = c_lo; c < c_lo + nc; ++c)
+            most = a.groups.out_count[c] > most ? a.groups.out_count[c] : most;
+        if (most > 1) {
+            using G = C2RGroups<LOGN>;
+            const int ng = most < kMaxGroups ? most : kMaxGroups;
+            CUtensorMap umap;
+            const cudaError_t e = encode_u_map(&umap, a.U, G::N, a.K, G::RB);
+            if (e != cudaSuccess) return e;
+            return launch_pdl(k_row_c2r_groups<LOGN>, dim3(G::N / G::RB, nc), G::GT * ng,
+                              G::SMEM * ng, st, umap, a.A, a.tw, a.groups, a.gp, a.temp, a.err,
+                              c_lo);
+        }
+    }
     return launch_c2r_shape<LOGN, V, false>(a, c_lo, nc, st);
 }
 template <int LOGN, int V>
