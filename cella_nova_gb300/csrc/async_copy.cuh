@@ -56,6 +56,25 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
         : "memory");
 }
 
+// The same for data that nothing reads again before much else has passed
+// through L2: its lines are the first to go.
+__device__ __forceinline__ void bulk_g2s_once(void* dst, const void* src, uint32_t bytes,
+                                              uint64_t* bar) {
+    uint64_t policy;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], "
+        "[%1], %2, [%3], %4;" ::"r"(smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
+        : "memory");
+}
+
+// Ask for `bytes` (a multiple of 16) from a 16-byte aligned address to be
+// brought into L2.
+__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 // 2-D tiled tensor copy global -> shared (TMA engine): the box of `map` at
 // element coordinates (x, y), x innermost, lands dense in shared memory and
 // completes on `bar`.  `map` is the address of a CUtensorMap in kernel

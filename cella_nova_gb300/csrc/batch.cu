@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(C2RShape<LOGN, V>::RT, C2RShape<LOGN, V>::MINB
 }
 
 template <int LOGN, int V>
-__global__ void __launch_bounds__(DiffTile<LOGN, V>::THREADS)
+__global__ void __launch_bounds__(DiffTile<LOGN, V>::THREADS, DiffTile<LOGN, V>::MINB)
     kb_diffusion(const WorldDesc* __restrict__ worlds, const WorkItem* __restrict__ items,
                  int count, int parity) {
     extern __shared__ __align__(128) float smb_diff[];
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(DiffTile<LOGN, V>::THREADS)
         const WorkItem it = items[i];
         const WorldDesc& w = worlds[it.world];
         diffusion_tile<LOGN, V>(w.A, w.state[parity], w.state[parity ^ 1], it.c, it.a, it.b,
-                                smb_diff, nullptr);
+                                smb_diff, nullptr, false);
     }
 }
 

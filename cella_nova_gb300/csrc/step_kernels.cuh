@@ -410,18 +410,26 @@ __device__ __forceinline__ bool col_conv_body(const float2* __restrict__ rowspec
     constexpr uint32_t kKernelBytes = KRE ? uint32_t(TW) * N * sizeof(float) : kTileBytes;
     const uint32_t q0 = phase;
     auto buffer = [&](uint32_t q) { return KS + (NBUF == 2 ? (q & 1u) * (TW * N) : 0); };
+    // From side 1024 on a step streams more than L2 holds: the row spectra are
+    // dead once read and the kernel spectra come round a whole step later, so
+    // both leave L2 first and U, A and the state stay longer (2048^2, C=3,
+    // K=9: 151 -> 148 us per step; C=1, K=1: 42.4 -> 40.7 us).
+    auto copy_tile = [&](float2* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+        if constexpr (G::SMALL) bulk_g2s(dst, src, bytes, bar);
+        else bulk_g2s_once(dst, src, bytes, bar);
+    };
     auto issue = [&](int stage) {   // thread 0 copies, after a barrier that closed the buffer's reads
         if (threadIdx.x != 0) return;
         uint64_t* bar = barp + (NBUF == 2 ? (q0 + stage) & 1u : 0);
         float2* dst = buffer(q0 + stage);
         if (stage == 0) {
             mbar_arrive_expect_tx(bar, kTileBytes);
-            bulk_g2s(dst, rowspec + (size_t(c) * M + kx0) * N, kTileBytes, bar);
+            copy_tile(dst, rowspec + (size_t(c) * M + kx0) * N, kTileBytes, bar);
         } else {
             const size_t off = (size_t(groups.in_idx[base + stage - 1]) * (M + 1) + kx0) * N;
             mbar_arrive_expect_tx(bar, kKernelBytes);
-            if constexpr (KRE) bulk_g2s(dst, kre + off, kKernelBytes, bar);
-            else bulk_g2s(dst, kspec + off, kKernelBytes, bar);
+            if constexpr (KRE) copy_tile(dst, kre + off, kKernelBytes, bar);
+            else copy_tile(dst, kspec + off, kKernelBytes, bar);
         }
     };
     auto issue_next = [&](int stage) {   // all threads call, after reading stage - NBUF
@@ -1192,15 +1200,21 @@ __device__ __forceinline__ void diffusion_pair_body(const float* __restrict__ A,
 }
 
 // The same arithmetic without shared memory: a thread owns 4 adjacent columns
-// and walks down TYR rows.  Per row it loads A at its columns +-2 and the
-// state at +-1 with three 16-byte loads each (the side ones overlap its
-// neighbours' and hit L1), splits A into heads and tails, and keeps the
-// horizontal 3-sums of the last three rows (heads, tails, q) in registers;
-// the vertical sums come from those slots.  Every sum keeps the order of
-// diffusion2_body, so the bits are the same.  A CTA is RS strips of TX/4
-// threads: TX columns by RS * TYR rows.  Strips of STRIP rows (variant 1:
+// and walks down TYR rows.  Per row it loads A at its columns -2 .. +5 and
+// the state at -1 .. +4 (16 bytes for its own columns; the side values
+// overlap its neighbours' and hit L1), splits A into heads and tails, and
+// keeps the horizontal 3-sums of the last three rows (heads, tails, q) in
+// registers; the vertical sums come from those slots.  Every sum keeps the
+// order of diffusion2_body, so the bits are the same.  A CTA is RS strips of
+// TX/4 threads: TX columns by RS * TYR rows.  Strips of STRIP rows (variant 1:
 // 16, variant 3: 8; fewer at small sides) trade the four halo rows each
 // strip re-reads against twice the CTAs and half the unrolled body.
+//
+// What bounds it is the bytes in flight: with one row of loads ahead at 80
+// registers (six CTAs per SM) it ran at 35.0 us at 2048^2, C=3, in 16-row
+// strips and 39.2 us in 8-row strips (151 MB in and out); with three rows ahead
+// at 123 registers (four CTAs) at 31.3 and 33.5 us.  Two rows at 96 registers:
+// 34.3 and 33.4 us; four rows: 30.8 and 34.1 us.
 template <int LOGN, int STRIP = 16>
 struct DiffGeoReg {
     static constexpr int N = 1 << LOGN;
@@ -1216,7 +1230,7 @@ template <int LOGN, int STRIP>
 __device__ __forceinline__ void diffusion_reg_body(const float* __restrict__ A,
                                                    const float* __restrict__ x,
                                                    float* __restrict__ out, int c, int x0,
-                                                   int y0, unsigned char* levels) {
+                                                   int y0, unsigned char* levels, bool ahead) {
     using D = DiffGeoReg<LOGN, STRIP>;
     constexpr int N = D::N, MASK = N * N - 1;
     const int col = x0 + 4 * (threadIdx.x % (D::TX / 4));   // first of this thread's columns
@@ -1224,15 +1238,28 @@ __device__ __forceinline__ void diffusion_reg_body(const float* __restrict__ A,
     const float* Ac = A + size_t(c) * N * N;
     const float* xc = x + size_t(c) * N * N;
     float* oc = out + size_t(c) * N * N;
-    const int cl = (col - 4) & (N - 1), cr = (col + 4) & (N - 1);
     unsigned char* lv = levels ? levels + size_t(c) * N * N : nullptr;
     const bool draw = levels != nullptr && c < 3;
-    // columns col-4 .. col+7 of row y (toroidal)
-    auto ld3 = [&](const float* p, int y, float4& l, float4& m, float4& r) {
-        const float* row = p + ((y * N) & MASK);
-        l = __ldg(reinterpret_cast<const float4*>(row + cl));
-        m = __ldg(reinterpret_cast<const float4*>(row + col));
-        r = __ldg(reinterpret_cast<const float4*>(row + cr));
+    // A at columns col-2 .. col+5 and the state at col-1 .. col+4 of a row
+    // (toroidal); the side values by 8- and 4-byte loads
+    struct RowA { float2 l; float4 m; float2 r; };
+    struct RowX { float l; float4 m; float r; };
+    const int l2 = (col - 2) & (N - 1), l1 = (col - 1) & (N - 1), rr = (col + 4) & (N - 1);
+    auto lda = [&](int y) {
+        const float* row = Ac + ((y * N) & MASK);
+        RowA v;
+        v.l = __ldg(reinterpret_cast<const float2*>(row + l2));
+        v.m = __ldg(reinterpret_cast<const float4*>(row + col));
+        v.r = __ldg(reinterpret_cast<const float2*>(row + rr));
+        return v;
+    };
+    auto ldx = [&](int y) {
+        const float* row = xc + ((y * N) & MASK);
+        RowX v;
+        v.l = __ldg(row + l1);
+        v.m = __ldg(reinterpret_cast<const float4*>(row + col));
+        v.r = __ldg(row + rr);
+        return v;
     };
 
     // slot k % 3 holds the sums of iteration k: heads / tails over Z columns
@@ -1240,20 +1267,37 @@ __device__ __forceinline__ void diffusion_reg_body(const float* __restrict__ A,
     // A at the output columns (am)
     float hs[3][6], ls[3][6], qs[3][4];
     float4 am[3];
-    // the loads of the next row are issued before this row's arithmetic
-    float4 nal, nac, nar;
-    float4 nxl = make_float4(0.f, 0.f, 0.f, 0.f), nxm = nxl, nxr = nxl;
-    ld3(Ac, ys - 2, nal, nac, nar);
+    // the loads of the next PF rows are in flight during this row's
+    // arithmetic (slot: row modulo PF)
+    constexpr int PF = 3, ITER = D::TYR + 4;
+    RowA na[PF];
+    RowX nx[PF];   // state row ya - 1 of iteration k >= 2
+    // A strip is a warp: its rows are asked into L2 together, the DRAM latency
+    // of all but the first then lies before they are needed
+    if (ahead && D::TX == 128) {
+        const int lane = threadIdx.x % 32;
+        if (lane < D::TYR + 4) prefetch_l2(Ac + (((ys - 2 + lane) * N) & MASK) + x0, 512);
+        if (lane < D::TYR + 2) prefetch_l2(xc + (((ys - 1 + lane) * N) & MASK) + x0, 512);
+    }
 #pragma unroll
-    for (int k = 0; k < D::TYR + 4; ++k) {
+    for (int i = 0; i < PF; ++i) {
+        na[i] = lda(ys - 2 + i);
+        if (i >= 2) nx[i] = ldx(ys - 3 + i);
+    }
+#pragma unroll
+    for (int k = 0; k < ITER; ++k) {
         const int ya = ys - 2 + k;   // A row of this iteration
         const int b = k % 3;
-        const float4 al = nal, ac = nac, ar = nar;
-        const float4 xl = nxl, xm = nxm, xr = nxr;   // state row ya - 1 (k >= 2)
-        if (k + 1 < D::TYR + 4) ld3(Ac, ya + 1, nal, nac, nar);
-        if (k + 1 >= 2 && k + 1 < D::TYR + 4) ld3(xc, ya, nxl, nxm, nxr);
+        const RowA av = na[k % PF];
+        const float4 ac = av.m;
+        RowX xr;
+        if (k >= 2) xr = nx[k % PF];
+        if (k + PF < ITER) {
+            na[k % PF] = lda(ya + PF);
+            if (k + PF >= 2) nx[k % PF] = ldx(ya + PF - 1);
+        }
         {
-            const float a[8] = {al.z, al.w, ac.x, ac.y, ac.z, ac.w, ar.x, ar.y};
+            const float a[8] = {av.l.x, av.l.y, ac.x, ac.y, ac.z, ac.w, av.r.x, av.r.y};
             float H[8], L[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -1269,7 +1313,7 @@ __device__ __forceinline__ void diffusion_reg_body(const float* __restrict__ A,
         }
         if (k >= 2) {   // Z and q at row ya - 1
             const int t0 = (k - 2) % 3, t1 = (k - 1) % 3;
-            const float xv[6] = {xl.w, xm.x, xm.y, xm.z, xm.w, xr.x};
+            const float xv[6] = {xr.l, xr.m.x, xr.m.y, xr.m.z, xr.m.w, xr.r};
             float q[6];
 #pragma unroll
             for (int j = 0; j < 6; ++j) {
@@ -1299,13 +1343,11 @@ __device__ __forceinline__ void diffusion_reg_body(const float* __restrict__ A,
 
 // The diffusion phase's variants: 1 and 3 the register body in 16- and 8-row
 // strips, 2 the column-pair body, 0 the shared-memory tile body up to side
-// 512 (at 256^2 2.5 us, against 7.0 and 4.1 us for the strips, whose rows
-// wait for their loads one after another) and the register body from 1024
-// on: there launch_diff takes 16-row strips where their CTAs fill the GPU at
-// least once and 8-row strips otherwise (2048^2: 35.0 against 39.2 us with
-// three channels, 15.6 against 10.6 us with one; 1024^2, C=3: 9.5 against
-// 9.1 us).  All give the same bits.  TX x TY is the tile of one CTA (one
-// work item).
+// 512 (at 256^2 2.4 us, against 6.6 and 4.0 us for the strips, whose rows
+// wait for their loads one after another) and the 8-row strips from 1024 on
+// (1024^2, C=3: 7.9 us, 9.2 us in 16 rows; 2048^2, C=1: both 9.1 us; C=3: 33.5
+// against 31.3 us alone, but 148.2 against 149.5 us for the whole step).  All
+// give the same bits.  TX x TY is the tile of one CTA (one work item).
 constexpr int kDiffVariants = 4;
 template <int LOGN, int V,
           int KIND = V == 2 ? 2 : (V == 1 || V == 3 || LOGN > kMaxSmallLogN) ? 1 : 0>
@@ -1313,7 +1355,9 @@ struct DiffTile;
 template <int LOGN, int V>
 struct DiffTile<LOGN, V, 1> {
     static constexpr bool REG = true, PAIR = false;
-    static constexpr int STRIP = (V == 3 || (V == 0 && LOGN == 10)) ? 8 : 16;
+    static constexpr int STRIP = (V == 1) ? 16 : 8;
+    // three rows of loads in flight take 123 registers: four CTAs per SM
+    static constexpr int MINB = 4;
     using D = DiffGeoReg<LOGN, STRIP>;
     static constexpr int THREADS = D::THREADS, TX = D::TX, TY = D::TY;
     static constexpr size_t SMEM = 0;
@@ -1322,14 +1366,14 @@ template <int LOGN, int V>
 struct DiffTile<LOGN, V, 2> {
     static constexpr bool REG = false, PAIR = true;
     using D = DiffGeoPair<LOGN, V>;
-    static constexpr int THREADS = D::THREADS, TX = D::TX, TY = D::TY;
+    static constexpr int THREADS = D::THREADS, TX = D::TX, TY = D::TY, MINB = 1;
     static constexpr size_t SMEM = D::SMEM;
 };
 template <int LOGN, int V>
 struct DiffTile<LOGN, V, 0> {
     static constexpr bool REG = false, PAIR = false;
     using D = DiffGeo2<LOGN, V>;
-    static constexpr int THREADS = D::THREADS, TX = D::TX, TY = D::TY;
+    static constexpr int THREADS = D::THREADS, TX = D::TX, TY = D::TY, MINB = 1;
     static constexpr size_t SMEM = D::SMEM;
 };
 
@@ -1337,10 +1381,10 @@ template <int LOGN, int V>
 __device__ __forceinline__ void diffusion_tile(const float* __restrict__ A,
                                                const float* __restrict__ x,
                                                float* __restrict__ out, int c, int x0, int y0,
-                                               float* smf, unsigned char* levels) {
+                                               float* smf, unsigned char* levels, bool ahead) {
     using T = DiffTile<LOGN, V>;
     if constexpr (T::REG)
-        diffusion_reg_body<LOGN, T::STRIP>(A, x, out, c, x0, y0, levels);
+        diffusion_reg_body<LOGN, T::STRIP>(A, x, out, c, x0, y0, levels, ahead);
     else if constexpr (T::PAIR)
         diffusion_pair_body<LOGN, V>(A, x, out, c, x0, y0, smf, levels);
     else
@@ -1348,14 +1392,14 @@ __device__ __forceinline__ void diffusion_tile(const float* __restrict__ A,
 }
 
 template <int LOGN, int V = 0>
-__global__ void __launch_bounds__(DiffTile<LOGN, V>::THREADS)
+__global__ void __launch_bounds__(DiffTile<LOGN, V>::THREADS, DiffTile<LOGN, V>::MINB)
     k_diffusion(const float* __restrict__ A, const float* __restrict__ x, float* __restrict__ out,
-                int cbase, unsigned char* __restrict__ levels) {
+                int cbase, unsigned char* __restrict__ levels, bool ahead) {
     extern __shared__ __align__(128) float sm_diff[];
     pdl_wait();
     pdl_launch_dependents();
     diffusion_tile<LOGN, V>(A, x, out, blockIdx.z + cbase, blockIdx.x * DiffTile<LOGN, V>::TX,
-                            blockIdx.y * DiffTile<LOGN, V>::TY, sm_diff, levels);
+                            blockIdx.y * DiffTile<LOGN, V>::TY, sm_diff, levels, ahead);
 }
 
 // ---------------------------------------------------------------------------
@@ -1664,18 +1708,22 @@ cudaError_t launch_c2r(const StepArgs& a, int c_lo, int nc, cudaStream_t st) {
     }
     return launch_c2r_shape<LOGN, V, false>(a, c_lo, nc, st);
 }
+// Whether a step's buffers (per grid point: the states, row spectra and A 16 B
+// per channel, both U and the spectra up to 12 B per kernel) outgrow L2, so
+// that the diffusion finds its inputs in DRAM.  With its rows asked into L2
+// ahead a step takes 151 instead of 153 us at 2048^2 with C=3, K=9 (352 MB at
+// least), 45.8 instead of 46.0 us at 1024^2, but 42.7 instead of 41.6 us at
+// 2048^2 with C=1, K=1 (117 MB).
+inline bool outgrows_l2(int n, int C, int K) {
+    return size_t(n) * n * (16 * size_t(C) + 12 * size_t(K)) > size_t(129) * 1000 * 1000;
+}
 template <int LOGN, int V>
 cudaError_t launch_diff(const StepArgs& a, int c_lo, int nc, cudaStream_t st) {
     constexpr int N = 1 << LOGN;
     using D = DiffTile<LOGN, V>;
-    if constexpr (V == 0 && D::REG) {
-        // all channels' CTAs of 16-row strips (six fit an SM's registers)
-        constexpr int kTiles = N / DiffTile<LOGN, 1>::TX * (N / DiffTile<LOGN, 1>::TY);
-        if (kTiles * a.C < 6 * 152) return launch_diff<LOGN, 3>(a, c_lo, nc, st);
-        return launch_diff<LOGN, 1>(a, c_lo, nc, st);
-    }
     return launch_pdl(k_diffusion<LOGN, V>, dim3(N / D::TX, N / D::TY, nc), D::THREADS,
-                      D::SMEM, st, a.A, a.x_in, a.x_out, c_lo, a.levels);
+                      D::SMEM, st, a.A, a.x_in, a.x_out, c_lo, a.levels,
+                      outgrows_l2(N, a.C, a.K));
 }
 
 #define CG_VARIANT_SWITCH(v, FN, ...)            \
