@@ -202,6 +202,53 @@ __device__ __forceinline__ void gather_rows(const float2* __restrict__ src, floa
     __syncthreads();
 }
 
+// The rows by 2-D tensor copies into a landing tile (element (kx, s) at
+// kx * RB + s, as in row_c2r_growth_body): the transpose of gather_rows costs
+// eight shared-memory wavefronts per 32 values, a sixth of the growth
+// adjoint's, where the copy engine does it for none.  Taken where the CTAs
+// outnumber their places (rows_landed), so that others cover the copy: a
+// gradient pass at 2048^2, C=2, K=4, 8 steps, 4485 -> 4133 us, at 1024^2, C=3,
+// K=9, 16 steps, 4197 -> 4127 us; with one channel and kernel at 1024^2 it
+// would take 1588 instead of 1544 us.  `plane` is the tile's plane of [M][N] in
+// the map.  Issue and wait; false (and *err) on
+// a bounded wait that timed out, for every thread alike.
+template <class G>
+__device__ __forceinline__ bool land_rows(const CUtensorMap* map, int plane, int y0, float2* land,
+                                          uint64_t* bar, int* err) {
+    if (threadIdx.x == 0) {
+        mbar_arrive_expect_tx(bar, uint32_t(G::C2R_TILE) * sizeof(float2));
+#pragma unroll
+        for (int q = 0; q < G::M / G::UBOX; ++q)
+            tensor2d_g2s(land + q * G::UBOX * G::RB, map, 2 * y0, plane * G::M + q * G::UBOX, bar);
+    }
+    const bool ok = mbar_wait(bar, 0, err);
+    if (!__syncthreads_or(!ok)) return true;
+    mbar_wait(bar, 0, nullptr);   // one more bounded chance to land before the CTA leaves
+    return false;
+}
+
+// Inverse row FFT of the RB packed rows in the landing tile, through the work
+// rows `buf`, the row index fastest over the threads; `out` as below.
+template <class G, class OUT>
+__device__ __forceinline__ void c2r_landed(const float2* land, float2* buf,
+                                           const float2* __restrict__ tw, OUT& out) {
+    SmemRows rows{buf, G::RP};
+    const float2* lt = land + threadIdx.x % G::RB;
+    auto ld0 = [&](int, int m, int, int q) -> float2 {
+        if (q == 0 && m == 0) {
+            const float2 x = lt[0];
+            return make_float2(x.x + x.y, x.x - x.y);
+        }
+        const float2 a = lt[m * G::RB];
+        const float2 b = cconj(lt[(G::M - m) * G::RB]);
+        const float2 E = cadd(a, b);
+        const float2 O = cmulc(csub(a, b), __ldg(&tw[m]));
+        return make_float2(E.x - O.y, E.y + O.x);
+    };
+    auto st = [&](int s, int i, float2 v, int, int) { out(s, i, v); };
+    FftPasses<G::M, 1, true, G::RT, G::RB, false, G::ROW_MR, true, false, true>::run(
+        ld0, rows, rows, st, tw + G::TW_ROW);
+}
 // Inverse row FFT of RB packed rows in `buf`; `out(s, i, v)` receives the
 // pixel pair (x[2i], x[2i+1]) of row s.
 template <class G, class OUT>
@@ -267,8 +314,9 @@ struct ChainedRows {
     }
 };
 
-template <int LOGN, int V = 0>
-__device__ __forceinline__ void growth_bwd_body(float2* __restrict__ U,
+template <int LOGN, int V, bool LAND>
+__device__ __forceinline__ void growth_bwd_body(const CUtensorMap* umap, uint64_t* bar, int* err,
+                                                float2* __restrict__ U,
                                                 const float* __restrict__ abar,
                                                 const float2* __restrict__ tw,
                                                 const AdjointParams& ap, int k, int cout,
@@ -284,7 +332,11 @@ __device__ __forceinline__ void growth_bwd_body(float2* __restrict__ U,
         else return RowsInOrder{};
     }();
     float2* Uk = U + size_t(k) * G::M * G::N + y0;
-    gather_rows<G>(Uk, sm, row);
+    if constexpr (LAND) {
+        if (!land_rows<G>(umap, k, y0, sm + G::C2R_LAND, bar, err)) return;
+    } else {
+        gather_rows<G>(Uk, sm, row);
+    }
     const float mu = ap.mu[k], w = ap.w[k], is2 = ap.inv_s2[k], is3 = ap.inv_s3[k];
     const float* ab = abar + (size_t(cout) * G::N + y0) * G::N;
     float pw = 0.f, pmu = 0.f, psg = 0.f;
@@ -305,9 +357,11 @@ __device__ __forceinline__ void growth_bwd_body(float2* __restrict__ U,
         }
         sm[s * G::RP + pidx(i)] = make_float2(ub[0], ub[1]);
     };
-    c2r_rows<G>(sm, tw, out);
+    if constexpr (LAND) c2r_landed<G>(sm + G::C2R_LAND, sm, tw, out);
+    else c2r_rows<G>(sm, tw, out);
     SmemRows rows{sm, G::RP};
-    FftPasses<G::M, 1, false, G::RT, G::RB, false, G::ROW_MR>::run(rows, rows, rows, rows, tw + G::TW_ROW);
+    FftPasses<G::M, 1, false, G::RT, G::RB, false, G::ROW_MR, LAND>::run(
+        rows, rows, rows, rows, tw + G::TW_ROW);
     r2c_finish<G>(sm, tw, Uk, row);
     const double sw = block_sum(double(pw), red);
     const double smu = block_sum(double(pmu), red);
@@ -319,18 +373,21 @@ __device__ __forceinline__ void growth_bwd_body(float2* __restrict__ U,
     }
 }
 
-template <int LOGN, int V = 0>
+template <int LOGN, int V = 0, bool LAND = false>
 __global__ void __launch_bounds__(GrowthRows<LOGN, V>::RT, 512 / GrowthRows<LOGN, V>::RT)
-    k_growth_bwd(float2* __restrict__ U, const float* __restrict__ abar,
-                 const float2* __restrict__ tw, const AdjointParams* __restrict__ app,
-                 double* __restrict__ pgrad, int K, int stride) {
+    k_growth_bwd(const __grid_constant__ CUtensorMap umap, float2* __restrict__ U,
+                 const float* __restrict__ abar, const float2* __restrict__ tw,
+                 const AdjointParams* __restrict__ app, double* __restrict__ pgrad, int K,
+                 int stride, int* err) {
     extern __shared__ __align__(128) float2 sm_gbwd[];
     __shared__ double red[16];
+    __shared__ __align__(8) uint64_t bar;
+    if constexpr (LAND) init_tile_barrier(&bar);
     pdl_wait();
     pdl_launch_dependents();
     const int k = blockIdx.y;
-    growth_bwd_body<LOGN, V>(U, abar, tw, *app, k, app->cout[k], blockIdx.x, stride, pgrad, K,
-                             sm_gbwd, red);
+    growth_bwd_body<LOGN, V, LAND>(&umap, &bar, err, U, abar, tw, *app, k, app->cout[k], blockIdx.x,
+                             stride, pgrad, K, sm_gbwd, red);
 }
 
 // ---------------------------------------------------------------------------
@@ -560,17 +617,24 @@ __global__ void __launch_bounds__(Geo<LOGN, V>::CT,
 // 5. Inverse row FFT of RB rows of a kx-major spectrum, scaled, written to
 //    (or added to) a real [C or K][n][n] array.  grid (N/RB, planes), RT.
 // ---------------------------------------------------------------------------
-template <int LOGN, int V = 0>
-__global__ void __launch_bounds__(Geo<LOGN, V>::RT, 512 / Geo<LOGN, V>::RT) k_row_c2r_add(const float2* __restrict__ src,
+template <int LOGN, int V = 0, bool LAND = false>
+__global__ void __launch_bounds__(Geo<LOGN, V>::RT, 512 / Geo<LOGN, V>::RT) k_row_c2r_add(const __grid_constant__ CUtensorMap smap,
+                                                      const float2* __restrict__ src,
                                                       float* __restrict__ dst,
                                                       const float2* __restrict__ tw, float scale,
-                                                      int accumulate) {
+                                                      int accumulate, int* err) {
     using G = Geo<LOGN, V>;
     extern __shared__ __align__(128) float2 sm_c2ra[];
+    __shared__ __align__(8) uint64_t bar;
+    if constexpr (LAND) init_tile_barrier(&bar);
     pdl_wait();
     pdl_launch_dependents();
     const int c = blockIdx.y, y0 = blockIdx.x * G::RB;
-    gather_rows<G>(src + size_t(c) * G::M * G::N + y0, sm_c2ra);
+    if constexpr (LAND) {
+        if (!land_rows<G>(&smap, c, y0, sm_c2ra + G::C2R_LAND, &bar, err)) return;
+    } else {
+        gather_rows<G>(src + size_t(c) * G::M * G::N + y0, sm_c2ra);
+    }
     float* d = dst + (size_t(c) * G::N + y0) * G::N;
     auto out = [&](int s, int i, float2 v) {
         float2* p = reinterpret_cast<float2*>(d + size_t(s) * G::N) + i;
@@ -582,7 +646,8 @@ __global__ void __launch_bounds__(Geo<LOGN, V>::RT, 512 / Geo<LOGN, V>::RT) k_ro
         }
         *p = o;
     };
-    c2r_rows<G>(sm_c2ra, tw, out);
+    if constexpr (LAND) c2r_landed<G>(sm_c2ra + G::C2R_LAND, sm_c2ra, tw, out);
+    else c2r_rows<G>(sm_c2ra, tw, out);
 }
 
 // Plain inverse column FFT of a kx-major [planes][M][N] spectrum, in place.
@@ -603,18 +668,36 @@ __global__ void __launch_bounds__(Geo<LOGN, V>::CT) k_col_inv(float2* __restrict
 // ---------------------------------------------------------------------------
 // Launchers.
 // ---------------------------------------------------------------------------
+// Shared memory of a row kernel: the work rows, and the landing tile.
+template <class G, bool LAND>
+constexpr size_t adj_row_smem() {
+    return LAND ? (size_t(G::C2R_LAND) + G::C2R_TILE) * sizeof(float2) : G::R2C_SMEM;
+}
+// Whether the row kernels over `planes` planes land their rows (land_rows):
+// sides from 1024 on, and more CTAs than the four per SM that fit.
+template <int LOGN>
+constexpr bool kMayLand = LOGN > kMaxSmallLogN;
+inline bool rows_landed(int ctas) { return ctas > 4 * 152; }
+
 template <int LOGN, int V>
 cudaError_t prepare_backward_variant() {
     using G = Geo<LOGN, V>;
     cudaError_t e;
-    const void* fns[5] = {reinterpret_cast<const void*>(k_diffusion_bwd<LOGN, V>),
+    const void* fns[7] = {reinterpret_cast<const void*>(k_diffusion_bwd<LOGN, V>),
                           reinterpret_cast<const void*>(k_growth_bwd<LOGN, V>),
                           reinterpret_cast<const void*>(k_col_conv_adj<LOGN, V>),
                           reinterpret_cast<const void*>(k_row_c2r_add<LOGN, V>),
-                          reinterpret_cast<const void*>(k_col_inv<LOGN, V>)};
-    const size_t smem[5] = {DiffBwdGeo<LOGN, V>::SMEM, GrowthRows<LOGN, V>::R2C_SMEM, AdjColGeo<LOGN, V>::SMEM,
-                            G::R2C_SMEM, size_t(G::TW) * G::CP * sizeof(float2)};
-    for (int i = 0; i < 5; ++i)
+                          reinterpret_cast<const void*>(k_col_inv<LOGN, V>),
+                          reinterpret_cast<const void*>(k_growth_bwd<LOGN, V, kMayLand<LOGN>>),
+                          reinterpret_cast<const void*>(k_row_c2r_add<LOGN, V, kMayLand<LOGN>>)};
+    const size_t smem[7] = {DiffBwdGeo<LOGN, V>::SMEM,
+                            GrowthRows<LOGN, V>::R2C_SMEM,
+                            AdjColGeo<LOGN, V>::SMEM,
+                            G::R2C_SMEM,
+                            size_t(G::TW) * G::CP * sizeof(float2),
+                            adj_row_smem<GrowthRows<LOGN, V>, kMayLand<LOGN>>(),
+                            adj_row_smem<G, kMayLand<LOGN>>()};
+    for (int i = 0; i < 7; ++i)
         if ((e = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       int(smem[i]))) != cudaSuccess)
             return e;
@@ -649,8 +732,19 @@ cudaError_t launch_diff_bwd(const BwdArgs& a, cudaStream_t st) {
 template <int LOGN, int V>
 cudaError_t launch_growth_bwd(const BwdArgs& a, cudaStream_t st) {
     using G = GrowthRows<LOGN, V>;
-    return launch_pdl(k_growth_bwd<LOGN, V>, dim3(G::N / G::RB, a.K), G::RT, G::R2C_SMEM, st,
-                      a.U, a.abar, a.tw, a.ap, a.pgrad, a.K, a.var.chosen ? 8 : 32);
+    const dim3 grid(G::N / G::RB, a.K);
+    const int stride = a.var.chosen ? 8 : 32;
+    CUtensorMap umap{};
+    if constexpr (kMayLand<LOGN>) {
+        if (rows_landed(grid.x * grid.y)) {
+            const cudaError_t e = encode_u_map(&umap, a.U, G::N, a.K, G::RB);
+            if (e != cudaSuccess) return e;
+            return launch_pdl(k_growth_bwd<LOGN, V, true>, grid, G::RT, adj_row_smem<G, true>(),
+                              st, umap, a.U, a.abar, a.tw, a.ap, a.pgrad, a.K, stride, a.err);
+        }
+    }
+    return launch_pdl(k_growth_bwd<LOGN, V>, grid, G::RT, G::R2C_SMEM, st, umap, a.U, a.abar, a.tw,
+                      a.ap, a.pgrad, a.K, stride, a.err);
 }
 template <int LOGN, int V>
 cudaError_t launch_col_adj(const BwdArgs& a, cudaStream_t st) {
@@ -662,8 +756,19 @@ cudaError_t launch_col_adj(const BwdArgs& a, cudaStream_t st) {
 template <int LOGN, int V>
 cudaError_t launch_c2r_add(const BwdArgs& a, cudaStream_t st) {
     using G = Geo<LOGN, V>;
-    return launch_pdl(k_row_c2r_add<LOGN, V>, dim3(G::N / G::RB, a.C), G::RT, G::R2C_SMEM, st,
-                      static_cast<const float2*>(a.rowspec), a.xbar, a.tw, 1.f, 1);
+    const dim3 grid(G::N / G::RB, a.C);
+    const float2* src = a.rowspec;
+    CUtensorMap smap{};
+    if constexpr (kMayLand<LOGN>) {
+        if (rows_landed(grid.x * grid.y)) {
+            const cudaError_t e = encode_u_map(&smap, src, G::N, a.C, G::RB);
+            if (e != cudaSuccess) return e;
+            return launch_pdl(k_row_c2r_add<LOGN, V, true>, grid, G::RT, adj_row_smem<G, true>(),
+                              st, smap, src, a.xbar, a.tw, 1.f, 1, a.err);
+        }
+    }
+    return launch_pdl(k_row_c2r_add<LOGN, V>, grid, G::RT, G::R2C_SMEM, st, smap, src, a.xbar,
+                      a.tw, 1.f, 1, a.err);
 }
 
 template <int LOGN>
@@ -709,12 +814,26 @@ cudaError_t launch_backward(const BwdArgs& a, cudaStream_t st) {
 // (kgrad is transformed in place).
 template <int LOGN>
 cudaError_t launch_kgrad_final(float2* kgrad, float* hbar, int K, const float2* tw,
-                               cudaStream_t st) {
+                               int* err, cudaStream_t st) {
     using G = Geo<LOGN>;
     k_col_inv<LOGN, 0><<<dim3(G::M / G::TW, K), G::CT, size_t(G::TW) * G::CP * sizeof(float2), st>>>(
         kgrad, tw);
-    k_row_c2r_add<LOGN, 0><<<dim3(G::N / G::RB, K), G::RT, G::R2C_SMEM, st>>>(
-        kgrad, hbar, tw, 1.f / (4.f * float(G::N) * float(G::N)), 0);
+    const dim3 grid(G::N / G::RB, K);
+    const float scale = 1.f / (4.f * float(G::N) * float(G::N));
+    CUtensorMap smap{};
+    bool landed = false;
+    if constexpr (kMayLand<LOGN>) {
+        landed = rows_landed(grid.x * grid.y);
+        if (landed) {
+            const cudaError_t e = encode_u_map(&smap, kgrad, G::N, K, G::RB);
+            if (e != cudaSuccess) return e;
+            k_row_c2r_add<LOGN, 0, true><<<grid, G::RT, adj_row_smem<G, true>(), st>>>(
+                smap, kgrad, hbar, tw, scale, 0, err);
+        }
+    }
+    if (!landed)
+        k_row_c2r_add<LOGN, 0><<<grid, G::RT, G::R2C_SMEM, st>>>(smap, kgrad, hbar, tw, scale, 0,
+                                                                 err);
     return cudaGetLastError();
 }
 

@@ -164,7 +164,7 @@ typedef cudaError_t (*launch_step_channel_fn)(const StepArgs&, int phases, int c
 typedef cudaError_t (*kspec_cols_fn)(const float2* rows, float2* kspec, const float2* tw,
                                       const double* zsum, int K, cudaStream_t);
 typedef cudaError_t (*kgrad_final_fn)(float2* kgrad, float* hbar, int K, const float2* tw,
-                                      cudaStream_t);
+                                      int* err, cudaStream_t);
 
 struct SizeOps {
     launch_step_fn step;

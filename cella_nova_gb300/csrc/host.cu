@@ -1295,7 +1295,8 @@ int cg_kernel_grad_spatial(cg_sim* s, float* kgrad, float* hbar) {
     if (!aligned16(kgrad) || !aligned16(hbar)) return misaligned("cg_kernel_grad_spatial");
     int rc = ensure_backward(s);
     if (rc != CG_OK) return rc;
-    CG_CHECK(s->ops->kgrad_final(reinterpret_cast<float2*>(kgrad), hbar, s->K, s->tw, s->stream),
+    CG_CHECK(s->ops->kgrad_final(reinterpret_cast<float2*>(kgrad), hbar, s->K, s->tw, s->err,
+                                 s->stream),
              "finishing the kernel gradient");
     return CG_OK;
 }
