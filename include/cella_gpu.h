@@ -213,8 +213,9 @@ int cg_timed_iterate(cg_sim* sim, double ms[4]);
  *        agree with variants 0-2 to rounding (the same step error bar
  *        against FP64), not bit for bit.
  * Diffusion has variants 0-3; the other phases below side 512 have 0-2.
- * cg_autotune times every variant of every phase `reps` times on the live
- * handle (the state is not advanced), keeps the fastest per phase, then
+ * cg_autotune times every variant of every phase at least `reps` times, in
+ * three rounds, on the live handle (the state is not advanced), keeps the
+ * fastest per phase, then
  * picks the graph layout (cg_set_graph_layout) and re-captures the step
  * graphs.  ms_out[4 * CG_MAX_VARIANTS] (phase-major:
  * [row FFT v0..v4, column v0..v4, inverse row + growth v0..v4, diffusion
