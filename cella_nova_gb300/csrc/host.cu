@@ -1452,7 +1452,7 @@ int cg_autotune(cg_sim* s, int reps, double ms_out[4 * CG_MAX_VARIANTS], int cho
             *slot[p] = v;
             StepArgs a = s->args(s->cur, nullptr);
             a.var = var;
-            for (int q = 0; q < p; ++q)   // inputs of phase p
+            for (int q = 0; i == 0 && q < p; ++q)   // inputs of phase p
                 CG_CHECK(s->ops->step(a, phases[q], s->stream), "autotune prologue");
             CG_CHECK(s->ops->step(a, phases[p], s->stream), "autotune warm-up");
             CG_CHECK(cudaEventRecord(s->ev[0], s->stream), "cudaEventRecord");
