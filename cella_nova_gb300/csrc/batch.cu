@@ -238,6 +238,9 @@ struct cg_batch {
         float* kspec_re = nullptr;
         std::vector<uint8_t> kreal;   // per kernel: point-symmetric (cg_batch_set_kernel)
         std::vector<uint8_t> kset;    // per kernel: uploaded
+        bool real() const {   // its column pass reads real spectra (mode 1)
+            return std::all_of(kreal.begin(), kreal.end(), [](uint8_t r) { return r != 0; });
+        }
         float2* U = nullptr;
         float* A = nullptr;
         KernelGroups groups{};
@@ -366,9 +369,7 @@ StepArgs world_step_args(const cg_batch* b, int w, int parity, const Variants& v
     a.x_out = W.state[parity ^ 1];
     a.rowspec = W.rowspec;
     a.kspec = W.kspec;
-    bool real = true;
-    for (uint8_t r : W.kreal) real = real && r != 0;
-    a.kre = real ? W.kspec_re : nullptr;
+    a.kre = W.real() ? W.kspec_re : nullptr;
     a.U = W.U;
     a.A = W.A;
     a.tw = b->tw_by_logn[W.logn];
@@ -846,14 +847,19 @@ int cg_batch_set_kernel(cg_batch* b, int world, int k, const float* spec) {
         BCHECK(launch_real_parts(packed, W.kspec_re + size_t(k) * (half + W.n), half + W.n,
                                  b->stream),
                "keeping the real parts");
+    const bool was_real = W.real();
     W.kreal[size_t(k)] = real ? 1 : 0;
     bool all = true, complete = !b->graphs_ready;
     W.kset[size_t(k)] = 1;
     for (const auto& w : b->worlds) {
-        for (uint8_t r : w.kreal) all = all && r != 0;
+        all = all && w.real();
         for (uint8_t u : w.kset) complete = complete && u != 0;
     }
-    const bool changed = all != b->kreal_all;
+    // The graphs hold the form of the spectra (real or complex): the batch's in
+    // mode 0, each world's own in mode 1.
+    bool changed = all != b->kreal_all;
+    for (const auto& sc : b->classes)
+        changed = changed || (sc.logn == W.logn && sc.mode == 1 && W.real() != was_real);
     if (changed) {
         BCHECK(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
         b->kreal_all = all;
