@@ -25,10 +25,10 @@
 //      hbar_k = ubar (*) x(-.),
 //   5. k_row_c2r_add: the inverse row FFT of that, added to xbar.
 #pragma once
+#include "divisor.h"
 #include "step_kernels.cuh"
 
 namespace cg {
-
 
 // ---------------------------------------------------------------------------
 // 2. Diffusion backward (one channel tile per CTA).
@@ -36,30 +36,6 @@ namespace cg {
 // A and ybar (2-pixel halo) and the state (1-pixel halo) arrive by 16-byte
 // loads: their tiles reach 4 pixels past the tile on each side, so every
 // load stays aligned (n is a multiple of 4, also across the toroidal wrap).
-
-// Division of several numerators by one z, each correctly rounded as x / z
-// is: from the correctly rounded reciprocal r of z, q0 = fl(x r) is within an
-// ulp of x / z, and q0 + (x - q0 z) r with the exact remainder is its rounding
-// (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Dev. 34 (1990) 111-119).  One
-// reciprocal and three instructions per numerator instead of a division each.
-// Outside [2^-100, 2^100], where r or the remainder could leave the normal
-// range, it divides.
-struct Divisor {
-    float z, r;
-    bool plain;
-    __device__ __forceinline__ explicit Divisor(float d) : z(d) {
-        const float m = fabsf(d);
-        plain = !(m >= 7.8886091e-31f && m <= 1.2676506e30f);
-        r = __frcp_rn(d);
-    }
-    __device__ __forceinline__ float divide(float x) const {
-        if (plain) return x / z;
-        const float q0 = x * r;
-        return fmaf(fmaf(-q0, z, x), r, q0);
-    }
-};
-
 template <int LOGN, int V = 0>
 struct DiffBwdGeo {
     static constexpr int TX = Geo<LOGN, V>::TX, TY = Geo<LOGN, V>::TY;
