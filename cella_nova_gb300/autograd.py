@@ -248,11 +248,21 @@ class DiffusionLeniaGPU(torch.nn.Module):
                                          device=device)
         from .orchestrator import creature_ring_specs, ring_spec_array
         self.specs = ring_spec_array(creature_ring_specs(cr)[0])
-        self._ring_counts, self._ring_slots = None, None   # rings()
+        self._find_ring_slots()
 
     def kernels(self):
         """The spatial kernels (K, n, n) as differentiable torch ops (float64)."""
         return self.builder(list(self.ring_weights))
+
+    def _find_ring_slots(self):
+        """Where the concatenated ring weights go in the padded (K, 8) array.
+        Made outside inference mode, whatever the caller is in: training uses
+        it too."""
+        self._ring_counts = tuple(b.numel() for b in self.ring_weights)
+        with torch.inference_mode(False):
+            self._ring_slots = torch.tensor(
+                [k * _abi.MAX_RINGS + l for k, c in enumerate(self._ring_counts)
+                 for l in range(min(c, _abi.MAX_RINGS))], device=self.world.device)
 
     def rings(self):
         """Ring weights padded to (K, 8), differentiable."""
@@ -260,11 +270,10 @@ class DiffusionLeniaGPU(torch.nn.Module):
         # their backward were a fifth of a small creature's host time
         weights = list(self.ring_weights)
         counts = tuple(b.numel() for b in weights)
-        if counts != self._ring_counts:
-            self._ring_counts = counts
-            self._ring_slots = torch.tensor(
-                [k * _abi.MAX_RINGS + l for k, c in enumerate(counts) for l in range(c)],
-                device=self.world.device)
+        if counts != self._ring_counts:   # ring_weights were replaced
+            self._find_ring_slots()
+        if max(counts) > _abi.MAX_RINGS:
+            weights = [b[:_abi.MAX_RINGS] for b in weights]
         flat = torch.cat(weights)
         padded = flat.new_zeros(len(weights) * _abi.MAX_RINGS)
         return padded.index_copy(0, self._ring_slots, flat).view(-1, _abi.MAX_RINGS)
