@@ -188,10 +188,10 @@ class _UnrollRings(torch.autograd.Function):
         check(lib.cg_ring_weight_grad(world.h, ctypes.cast(ctx.specs, ctypes.c_void_p), _p(rw),
                                       _p(hbar), _p(grings)))
         ds, dm, dsg, dw, dr = ctx.dtypes
-        if dm == dsg == dw:   # one conversion for the three
-            pgrad = pgrad.to(dm)
-        return (None, None, None, None, g0.to(ds), pgrad[:K].to(dm), pgrad[K:2 * K].to(dsg),
-                pgrad[2 * K:].to(dw), grings.to(dr))
+        # copies: views of one storage would be saved with all of it and start
+        # at odd offsets
+        return (None, None, None, None, g0.to(ds), pgrad[:K].to(dm, copy=True),
+                pgrad[K:2 * K].to(dsg, copy=True), pgrad[2 * K:].to(dw, copy=True), grings.to(dr))
 
 
 def unroll_rings(world: LeniaWorld, specs, seed, mu, sigma, weights, rings, T: int,

@@ -1,4 +1,5 @@
-"""DiffusionLeniaGPU's padded ring weights."""
+"""DiffusionLeniaGPU's parameters: the padded ring weights, and gradients that
+are tensors of their own."""
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -45,6 +46,21 @@ def test_rings_of_other_counts(model):
         model.rings().sum().backward()
         assert torch.equal(model.ring_weights[1].grad, (weights <= MAX_RINGS).double())
     assert before.shape == (len(model.ring_weights), MAX_RINGS)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_gradients_share_no_storage(dtype):
+    m = autograd.DiffusionLeniaGPU(make_creature(64, 2, seed=6, radius=(4, 10), seed_box=32),
+                                   autotune=False)
+    leaves = [p.detach().to(dtype).requires_grad_() for p in (m.mu, m.sigma, m.weights)]
+    xT = autograd.unroll_rings(m.world, m.specs, m.seed, *leaves, m.rings(), 2, 2)
+    (xT ** 2).sum().backward()
+    for p in leaves:
+        g = p.grad
+        assert g.dtype == dtype and torch.isfinite(g).all()
+        assert g.untyped_storage().nbytes() == g.numel() * g.element_size()
+        assert g.storage_offset() == 0
 
 
 @pytest.mark.gpu
