@@ -266,27 +266,31 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // The rows of a CTA.  A thread adds its values to three FP32 sums before the
 // block adds the threads' sums in FP64, so which values share a thread decides
 // the parameter gradients' rounding.  At sides 64 to 256 a thread sums CHAIN
-// rows `stride` apart (32 where the world runs untuned, 8 where variants were
-// chosen), whatever the CTA shape: CTAs of 64 threads take 4 adjacent rows
-// of each of the CHAIN groups.  Elsewhere a thread's rows follow from the shape
-// (at 16, 32 and 512 a thread has one row's 16 values in every shape).
+// rows STRIDE apart in every variant: CTAs of 64 threads take 4 adjacent rows of
+// each of the CHAIN groups.  Elsewhere a thread's rows follow from the CTA shape
+// (at 16, 32 and 512 a thread has one row's 16 values in every shape) and, from
+// 1024 on, from how the rows arrive (land_rows).
 template <int LOGN, int V, bool CHAINED = (LOGN >= 6 && LOGN <= 8)>
 struct GrowthRows : Geo<LOGN, V> {
-    static constexpr int CHAIN = 1, GROUP = Geo<LOGN, V>::RB;
+    using Row = RowsInOrder;
+    __device__ __forceinline__ static int first(int block) { return block * Geo<LOGN, V>::RB; }
 };
 template <int LOGN, int V>
 struct GrowthRows<LOGN, V, true> : Geo<LOGN, V> {
     using G = Geo<LOGN, V>;
-    static constexpr int CHAIN = LOGN == 7 ? 4 : 2, GROUP = 4;
+    static constexpr int CHAIN = LOGN == 7 ? 4 : 2, GROUP = 4, STRIDE = 8;
     static constexpr int RB = GROUP * CHAIN, RT = 64;
     static constexpr int RP = padded_len(G::M) + (RB >= 16 ? 1 : 2);
     static constexpr size_t R2C_SMEM = size_t(RB) * RP * sizeof(float2);
     static_assert(GROUP * (G::M / last_radix(G::M)) == RT, "one group of rows per sweep");
-};
-struct ChainedRows {
-    int group, stride;
-    __device__ __forceinline__ int operator()(int s) const {
-        return s % group + s / group * stride;
+    struct Row {
+        __device__ __forceinline__ int operator()(int s) const {
+            return s % GROUP + s / GROUP * STRIDE;
+        }
+    };
+    __device__ __forceinline__ static int first(int block) {
+        constexpr int GROUPS = STRIDE / GROUP;   // CTAs per chain of rows
+        return block / GROUPS * (STRIDE * CHAIN) + block % GROUPS * GROUP;
     }
 };
 
@@ -296,17 +300,11 @@ __device__ __forceinline__ void growth_bwd_body(const CUtensorMap* umap, uint64_
                                                 const float* __restrict__ abar,
                                                 const float2* __restrict__ tw,
                                                 const AdjointParams& ap, int k, int cout,
-                                                int block, int stride, double* __restrict__ pgrad,
-                                                int K, float2* sm, double* red) {
+                                                int block, double* __restrict__ pgrad, int K,
+                                                float2* sm, double* red) {
     using G = GrowthRows<LOGN, V>;
-    constexpr bool CHAINED = G::CHAIN > 1;
-    const int groups = stride / G::GROUP;   // per chain
-    const int y0 = CHAINED ? block / groups * (stride * G::CHAIN) + block % groups * G::GROUP
-                           : block * G::RB;
-    const std::conditional_t<CHAINED, ChainedRows, RowsInOrder> row = [&] {
-        if constexpr (CHAINED) return ChainedRows{G::GROUP, stride};
-        else return RowsInOrder{};
-    }();
+    const int y0 = G::first(block);
+    const typename G::Row row;
     float2* Uk = U + size_t(k) * G::M * G::N + y0;
     if constexpr (LAND) {
         if (!land_rows<G>(umap, k, y0, sm + G::C2R_LAND, bar, err)) return;
@@ -354,7 +352,7 @@ __global__ void __launch_bounds__(GrowthRows<LOGN, V>::RT, 512 / GrowthRows<LOGN
     k_growth_bwd(const __grid_constant__ CUtensorMap umap, float2* __restrict__ U,
                  const float* __restrict__ abar, const float2* __restrict__ tw,
                  const AdjointParams* __restrict__ app, double* __restrict__ pgrad, int K,
-                 int stride, int* err) {
+                 int* err) {
     extern __shared__ __align__(128) float2 sm_gbwd[];
     __shared__ double red[16];
     __shared__ __align__(8) uint64_t bar;
@@ -363,7 +361,7 @@ __global__ void __launch_bounds__(GrowthRows<LOGN, V>::RT, 512 / GrowthRows<LOGN
     pdl_launch_dependents();
     const int k = blockIdx.y;
     growth_bwd_body<LOGN, V, LAND>(&umap, &bar, err, U, abar, tw, *app, k, app->cout[k], blockIdx.x,
-                             stride, pgrad, K, sm_gbwd, red);
+                                   pgrad, K, sm_gbwd, red);
 }
 
 // ---------------------------------------------------------------------------
@@ -709,18 +707,17 @@ template <int LOGN, int V>
 cudaError_t launch_growth_bwd(const BwdArgs& a, cudaStream_t st) {
     using G = GrowthRows<LOGN, V>;
     const dim3 grid(G::N / G::RB, a.K);
-    const int stride = a.var.chosen ? 8 : 32;
     CUtensorMap umap{};
     if constexpr (kMayLand<LOGN>) {
         if (rows_landed(grid.x * grid.y)) {
             const cudaError_t e = encode_u_map(&umap, a.U, G::N, a.K, G::RB);
             if (e != cudaSuccess) return e;
             return launch_pdl(k_growth_bwd<LOGN, V, true>, grid, G::RT, adj_row_smem<G, true>(),
-                              st, umap, a.U, a.abar, a.tw, a.ap, a.pgrad, a.K, stride, a.err);
+                              st, umap, a.U, a.abar, a.tw, a.ap, a.pgrad, a.K, a.err);
         }
     }
     return launch_pdl(k_growth_bwd<LOGN, V>, grid, G::RT, G::R2C_SMEM, st, umap, a.U, a.abar, a.tw,
-                      a.ap, a.pgrad, a.K, stride, a.err);
+                      a.ap, a.pgrad, a.K, a.err);
 }
 template <int LOGN, int V>
 cudaError_t launch_col_adj(const BwdArgs& a, cudaStream_t st) {

@@ -35,11 +35,6 @@ struct GrowthParams {
 // grid sides from 2^kMinPairLogN) change the FFT plans (step_kernels.cuh).
 struct Variants {
     int r2c = 0, col = 0, c2r = 0, diff = 0;
-    // Variants were chosen for this world (by the tuner or by hand).  The
-    // growth adjoint's FP32 partial sums follow it (GrowthRows), not the
-    // shape of any kernel, so that a kernel's CTA shape can change without
-    // changing the parameter gradients.
-    bool chosen = false;
 };
 constexpr int kMinPairLogN = 9;
 constexpr int kMaxSmallLogN = 9;   // sides whose phases take many small CTAs (Geo)

@@ -1412,7 +1412,6 @@ int cg_set_variants(cg_sim* s, const int v[4]) {
     s->var.col = v[1];
     s->var.c2r = v[2];
     s->var.diff = v[3];
-    s->var.chosen = true;
     return recapture(s);
 }
 
@@ -1478,7 +1477,6 @@ int cg_autotune(cg_sim* s, int reps, double ms_out[4 * CG_MAX_VARIANTS], int cho
     s->var.col = best[1];
     s->var.c2r = best[2];
     s->var.diff = best[3];
-    s->var.chosen = true;
     // then the graph layout: each layout's graph of kStepsPerGraph steps,
     // all reading the current state (nothing steps), replayed reps times
     double lay_ms[2] = {0.0, 0.0};
