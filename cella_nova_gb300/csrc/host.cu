@@ -209,6 +209,15 @@ struct HostPipe {
     bool ready = false;
 };
 
+// Steps per graph, and the graph of one step that also renders.  Between two
+// graphs the GPU drains and starts again (8-10 us at 512^2 with four channels,
+// against 26 us per step), so a count that is no multiple of eight takes
+// graphs of four and two before single steps.
+constexpr int kGraphs = 5;
+constexpr int kGraphSteps[kGraphs] = {8, 4, 2, 1, 1};
+constexpr int kStepsPerGraph = kGraphSteps[0];
+constexpr int kOneStep = 3, kRenderStep = 4;   // indexes of the last two
+
 struct cg_sim {
     int n = 0, logn = 0, C = 0, K = 0;
     float temp = 1.f;
@@ -227,10 +236,10 @@ struct cg_sim {
     float* kspec_re = nullptr;
     std::vector<uint8_t> kreal;
     bool kreal_all = false;
-    // kernels uploaded so far: with the last one the step graphs are captured
-    // (or with the first step), not at creation and again here
+    // kernels uploaded so far, and whether all have been: with the last one
+    // every step graph is captured
     std::vector<uint8_t> kset;
-    bool graphs_ready = false;
+    bool kset_all = false;
     float2* U = nullptr;       // two [K][n/2][n] buffers, one per ping-pong parity
     float* A = nullptr;
     float2* tw = nullptr;
@@ -238,8 +247,7 @@ struct cg_sim {
     double* mass_partial = nullptr;
     double* mass_out = nullptr;
     int* err = nullptr;   // device error word written by bounded waits
-    cudaGraphExec_t graph[4][2] = {};   // kGraphSteps[i] steps, per parity
-    cudaGraphExec_t graphR[2] = {nullptr, nullptr};    // one step that also renders
+    cudaGraphExec_t graph[kGraphs][2] = {};   // kGraphSteps[i] steps, per parity
     unsigned* render = nullptr;   // [n][n] packed 0x00RRGGBB
     unsigned char* levels = nullptr;   // [3][n][n] render levels of a rendering step
     unsigned char* frames[2] = {nullptr, nullptr};   // pinned RGB24 frames (frame streaming)
@@ -298,8 +306,6 @@ void release(cg_sim* s) {
     for (auto& per_parity : s->graph)
         for (auto& g : per_parity)
             if (g) cudaGraphExecDestroy(g);
-    for (auto& g : s->graphR)
-        if (g) cudaGraphExecDestroy(g);
     for (auto& e : s->ev)
         if (e) cudaEventDestroy(e);
     cudaFree(s->state[0]);
@@ -338,13 +344,6 @@ void release(cg_sim* s) {
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
     delete s;
 }
-
-// Steps per graph.  Between two graphs the GPU drains and starts again (8-10 us
-// at 512^2 with four channels, against 26 us per step), so a count that is
-// no multiple of eight takes graphs of four and two before single steps.
-constexpr int kGraphSteps[4] = {8, 4, 2, 1};
-constexpr int kStepsPerGraph = kGraphSteps[0];
-constexpr int kOneStep = 3;   // index of the one-step graph
 
 // Phases of a step in a chain of steps: where the world's diffusion takes the
 // next step's forward row pass with it (into a->rowspec_next, by default the
@@ -470,26 +469,43 @@ cudaError_t capture_steps(cg_sim* s, int p0, int nsteps, bool render, cudaGraphE
     return e;
 }
 
-void drop_graphs(cg_sim* s) {
-    for (auto* set : {s->graph[0], s->graph[1], s->graph[2], s->graph[3], s->graphR})
-        for (int p = 0; p < 2; ++p)
-            if (set[p]) {
-                cudaGraphExecDestroy(set[p]);
-                set[p] = nullptr;
-            }
+void drop_graph(cg_sim* s, int i, int p) {
+    if (s->graph[i][p]) cudaGraphExecDestroy(s->graph[i][p]);
+    s->graph[i][p] = nullptr;
 }
 
-int capture_graphs(cg_sim* s) {
-    s->graphs_ready = false;
-    drop_graphs(s);
-    for (int p = 0; p < 2; ++p) {
-        cudaError_t e = cudaSuccess;
-        for (int i = 0; i < 4 && e == cudaSuccess; ++i)
-            e = capture_steps(s, p, kGraphSteps[i], false, &s->graph[i][p]);
-        if (e == cudaSuccess) e = capture_steps(s, p, 1, true, &s->graphR[p]);
-        if (e != cudaSuccess) return cuda_fail(e, "capturing the step graph");
-    }
-    s->graphs_ready = true;
+int capture_graph(cg_sim* s, int i, int p) {
+    const cudaError_t e =
+        capture_steps(s, p, kGraphSteps[i], i == kRenderStep, &s->graph[i][p]);
+    return e == cudaSuccess ? CG_OK : cuda_fail(e, "capturing a step graph");
+}
+
+// The step graphs that are not there yet.
+int capture_missing(cg_sim* s) {
+    for (int i = 0; i < kGraphs; ++i)
+        for (int p = 0; p < 2; ++p)
+            if (!s->graph[i][p]) {
+                const int rc = capture_graph(s, i, p);
+                if (rc != CG_OK) return rc;
+            }
+    return CG_OK;
+}
+
+// The step graphs that are there, captured anew (none stays as it was, also
+// where a capture fails).
+int recapture(cg_sim* s) {
+    bool had[kGraphs][2];
+    for (int i = 0; i < kGraphs; ++i)
+        for (int p = 0; p < 2; ++p) {
+            had[i][p] = s->graph[i][p] != nullptr;
+            drop_graph(s, i, p);
+        }
+    for (int i = 0; i < kGraphs; ++i)
+        for (int p = 0; p < 2; ++p)
+            if (had[i][p]) {
+                const int rc = capture_graph(s, i, p);
+                if (rc != CG_OK) return rc;
+            }
     return CG_OK;
 }
 
@@ -542,21 +558,6 @@ int upload_params(cg_sim* s) {
     return CG_OK;
 }
 
-// Capture the step graphs anew, if they have been captured at all.
-int recapture(cg_sim* s) { return s->graphs_ready ? capture_graphs(s) : CG_OK; }
-
-// The step graphs, before a step is enqueued on st: captured now if they are
-// not yet.  Where st itself is being captured and they are not there, the
-// step's kernels go into that capture instead (*direct).
-int ensure_graphs(cg_sim* s, cudaStream_t st, bool* direct) {
-    *direct = false;
-    if (s->graphs_ready) return CG_OK;
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) cudaGetLastError();
-    *direct = status == cudaStreamCaptureStatusActive;
-    return *direct ? CG_OK : capture_graphs(s);
-}
-
 // One step's kernels straight into st (with render: the words as well).
 int step_direct(cg_sim* s, cudaStream_t st, bool render) {
     StepArgs a = s->args(s->cur, nullptr);
@@ -565,6 +566,27 @@ int step_direct(cg_sim* s, cudaStream_t st, bool render) {
     if (render)
         CG_CHECK(launch_pack_levels(s->levels, s->C, s->px(), s->render, st), "packing levels");
     s->cur ^= 1;
+    return CG_OK;
+}
+
+// kGraphSteps[i] steps on st by their graph.  One that is not there (a world
+// whose kernels were built on the device) is captured now, and only that one;
+// where st itself is being captured, the steps' kernels go into that capture.
+int step_by_graph(cg_sim* s, int i, cudaStream_t st) {
+    if (!s->graph[i][s->cur]) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &status) != cudaSuccess) cudaGetLastError();
+        int rc = CG_OK;
+        if (status == cudaStreamCaptureStatusActive) {
+            for (int t = 0; t < kGraphSteps[i] && rc == CG_OK; ++t)
+                rc = step_direct(s, st, i == kRenderStep);
+            return rc;
+        }
+        rc = capture_graph(s, i, s->cur);
+        if (rc != CG_OK) return rc;
+    }
+    CG_CHECK(cudaGraphLaunch(s->graph[i][s->cur], st), "cudaGraphLaunch");
+    s->cur ^= kGraphSteps[i] & 1;
     return CG_OK;
 }
 
@@ -733,24 +755,25 @@ namespace {
 // Record whether kernel k's spectrum is real (k < 0: every kernel not real);
 // when the world's column pass changes between the real and the complex
 // form, re-capture the step graphs; with the last kernel's first upload,
-// capture them.
+// capture those that are missing.
 int set_kernel_realness(cg_sim* s, int k, bool real) {
     if (k >= 0) s->kreal[size_t(k)] = real ? 1 : 0;
     else std::fill(s->kreal.begin(), s->kreal.end(), uint8_t(0));
     bool all = true;
     for (uint8_t r : s->kreal) all = all && r != 0;
-    bool complete = false;
-    if (k >= 0 && !s->graphs_ready) {
-        s->kset[size_t(k)] = 1;
-        complete = true;
-        for (uint8_t u : s->kset) complete = complete && u != 0;
-    }
-    if (all == s->kreal_all && !complete) return CG_OK;
     if (all != s->kreal_all) {
         CG_CHECK(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
         s->kreal_all = all;
+        const int rc = recapture(s);
+        if (rc != CG_OK) return rc;
     }
-    return complete ? capture_graphs(s) : recapture(s);
+    if (k < 0 || s->kset_all) return CG_OK;
+    s->kset[size_t(k)] = 1;
+    for (uint8_t u : s->kset)
+        if (u == 0) return CG_OK;
+    const int rc = capture_missing(s);
+    s->kset_all = rc == CG_OK;
+    return rc;
 }
 }  // namespace
 
@@ -816,20 +839,11 @@ int cg_upload_channel_f32(cg_sim* s, int c, const float* data) {
 int cg_step(cg_sim* s, int nsteps) {
     if (!s) return fail(CG_ERR_ARG, "cg_step: NULL handle");
     if (nsteps < 0) return fail(CG_ERR_ARG, "negative step count %d", nsteps);
-    bool direct = false;
-    if (nsteps > 0) {
-        const int rc = ensure_graphs(s, s->stream, &direct);
-        if (rc != CG_OK) return rc;
-    }
-    for (int i = 0; direct && i < nsteps; ++i) {
-        const int rc = step_direct(s, s->stream, false);
-        if (rc != CG_OK) return rc;
-    }
-    int left = direct ? 0 : nsteps;
-    for (int i = 0; i < 4; ++i)
+    int left = nsteps;
+    for (int i = 0; i <= kOneStep; ++i)
         for (; left >= kGraphSteps[i]; left -= kGraphSteps[i]) {
-            CG_CHECK(cudaGraphLaunch(s->graph[i][s->cur], s->stream), "cudaGraphLaunch");
-            s->cur ^= kGraphSteps[i] & 1;
+            const int rc = step_by_graph(s, i, s->stream);
+            if (rc != CG_OK) return rc;
         }
     return CG_OK;
 }
@@ -838,13 +852,7 @@ int cg_iterate(cg_sim* s) { return cg_step(s, 1); }
 
 int cg_iterate_and_render(cg_sim* s) {
     if (!s) return fail(CG_ERR_ARG, "cg_iterate_and_render: NULL handle");
-    bool direct = false;
-    const int rc = ensure_graphs(s, s->stream, &direct);
-    if (rc != CG_OK) return rc;
-    if (direct) return step_direct(s, s->stream, true);
-    CG_CHECK(cudaGraphLaunch(s->graphR[s->cur], s->stream), "cudaGraphLaunch");
-    s->cur ^= 1;
-    return CG_OK;
+    return step_by_graph(s, kRenderStep, s->stream);
 }
 
 int cg_render(cg_sim* s) {
@@ -940,14 +948,7 @@ int cg_render_ptr(cg_sim* s, const uint32_t** out) {
 
 int cg_iterate_on(cg_sim* s, cg_stream_t stream) {
     if (!s) return fail(CG_ERR_ARG, "cg_iterate_on: NULL handle");
-    cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : s->stream;
-    bool direct = false;
-    const int rc = ensure_graphs(s, st, &direct);
-    if (rc != CG_OK) return rc;
-    if (direct) return step_direct(s, st, false);
-    CG_CHECK(cudaGraphLaunch(s->graph[kOneStep][s->cur], st), "cudaGraphLaunch");
-    s->cur ^= 1;
-    return CG_OK;
+    return step_by_graph(s, kOneStep, stream ? static_cast<cudaStream_t>(stream) : s->stream);
 }
 
 int cg_download_channels(cg_sim* s, float* out) {
