@@ -506,6 +506,7 @@ cudaError_t enqueue_class_steps(cg_batch* b, const cg_batch::SizeClass& sc, int 
 // on a forked stream of its own: one class's phase tails overlap the other's
 // work.
 cudaError_t capture_batch_graphs(cg_batch* b) {
+    const OwnCapture own;
     b->graphs_ready = false;
     for (auto& per_parity : b->graph)
         for (auto& g : per_parity)

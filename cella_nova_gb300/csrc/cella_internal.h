@@ -80,6 +80,18 @@ struct StepArgs {
     Variants var;
 };
 
+// While one lives, this thread's calls may capture, instantiate and destroy
+// graphs of the library's own although a capture of the caller's is under way
+// (in this thread or, in global mode, in any): the step graphs' streams are
+// not part of it, and a refused call would end it.
+struct OwnCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OwnCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OwnCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    OwnCapture(const OwnCapture&) = delete;
+    OwnCapture& operator=(const OwnCapture&) = delete;
+};
+
 // Whether a world's diffusion can take the next step's forward row pass with
 // it: small sides, and a forward row pass of variants 0-2, whose bits it gives.
 inline bool fuses_next_row(int logn, const Variants& var) {

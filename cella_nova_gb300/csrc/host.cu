@@ -470,11 +470,13 @@ cudaError_t capture_steps(cg_sim* s, int p0, int nsteps, bool render, cudaGraphE
 }
 
 void drop_graph(cg_sim* s, int i, int p) {
+    const OwnCapture own;
     if (s->graph[i][p]) cudaGraphExecDestroy(s->graph[i][p]);
     s->graph[i][p] = nullptr;
 }
 
 int capture_graph(cg_sim* s, int i, int p) {
+    const OwnCapture own;
     const cudaError_t e =
         capture_steps(s, p, kGraphSteps[i], i == kRenderStep, &s->graph[i][p]);
     return e == cudaSuccess ? CG_OK : cuda_fail(e, "capturing a step graph");

@@ -1,5 +1,6 @@
 """The first steps of a world: its step graphs are captured as they are needed
-where its kernels were built on the device."""
+where its kernels were built on the device, and beside any capture of the
+caller's."""
 import time
 
 import numpy as np
@@ -7,7 +8,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from cella_nova_gb300 import GpuMaceLenia  # noqa: E402
+from cella_nova_gb300 import GpuMaceLenia, GpuMaceLeniaBatch  # noqa: E402
 from cella_nova_gb300.creature import make_creature  # noqa: E402
 from cella_nova_gb300.orchestrator import creature_ring_specs  # noqa: E402
 
@@ -68,3 +69,60 @@ def test_graphs_captured_on_demand_step_the_same(n):
             b.iterate()
         b.iterate_and_render()
         np.testing.assert_array_equal(a.state(), b.state())
+
+def test_first_step_beside_a_capture_on_another_stream():
+    cr = make_creature(128, 2, seed=1003, radius=(6, 16), seed_box=64)
+    st, x = torch.cuda.Stream(), torch.zeros(4, device="cuda")
+    with built_world(cr) as a, built_world(cr) as b:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            x += 1
+            a.run_steps(3)
+        b.run_steps(3)
+        np.testing.assert_array_equal(a.state(), b.state())
+        g.replay()
+        torch.cuda.synchronize()
+        assert x.tolist() == [1.0] * 4   # capturing runs nothing
+        np.testing.assert_array_equal(a.state(), b.state())   # the graph holds no step
+
+
+def test_last_kernel_set_under_capture():
+    """cg_set_kernel_device only enqueues work, also with the last kernel."""
+    cr = make_creature(128, 2, seed=1004, radius=(6, 16), seed_box=64)
+    spec = torch.view_as_real(torch.tensor(np.asarray(cr.kspec, np.complex64),
+                                           device="cuda")).contiguous()
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    with empty_world(cr, st.cuda_stream) as a, empty_world(cr) as b:
+        a.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            for k in range(cr.K):
+                a.set_kernel_device(spec[k].data_ptr(), k)
+        with torch.cuda.stream(st):
+            g.replay()
+        for k in range(cr.K):
+            b.set_kernel_device(spec[k].data_ptr(), k)
+        a.run_steps(5)
+        b.run_steps(5)
+        np.testing.assert_array_equal(a.state(), b.state())
+
+
+def test_first_batch_step_beside_a_capture():
+    """A batch that lacks a kernel captures its graphs with its first step."""
+    cr = make_creature(64, 2, seed=1005, radius=(4, 10), seed_box=32)
+
+    class Partial(GpuMaceLeniaBatch):
+        def set_kernel(self, world, k, spec):
+            if k > 0:
+                super().set_kernel(world, k, spec)
+
+    st, x = torch.cuda.Stream(), torch.zeros(4, device="cuda")
+    with Partial([cr, cr]) as a, Partial([cr, cr]) as b:
+        a.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            x += 1
+            a.run_steps(5)
+        b.run_steps(5)
+        np.testing.assert_array_equal(a.state(1), b.state(1))
