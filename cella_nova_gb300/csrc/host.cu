@@ -356,6 +356,9 @@ int chain_step(const cg_sim* s, StepArgs* a, bool after, bool before,
     return after ? kPhaseAll & ~kPhaseRowFwd : int(kPhaseAll);
 }
 
+// Whether the two graph layouts are different graphs (capture_steps).
+bool layouts_differ(const cg_sim* s) { return s->logn >= kMaxSmallLogN; }
+
 // Capture `nsteps` steps starting at ping-pong parity p0 as one graph whose
 // launches are per channel, on one stream per channel, so that independent
 // channels overlap (one channel's diffusion runs in another's tail).  Only
@@ -378,7 +381,7 @@ cudaError_t capture_steps(cg_sim* s, int p0, int nsteps, bool render, cudaGraphE
     // (64^2, C=3: 14.5 against 20.1 us for a one-step graph, 11.0 against
     // 13.4 us per step in a graph of eight; from 512^2 on the overlap wins,
     // 25.3 against 30.9 us).
-    if (s->layout == 1 || s->logn < kMaxSmallLogN) {
+    if (s->layout == 1 || !layouts_differ(s)) {
         cudaStream_t st0 = nullptr;
         cudaError_t e = cudaStreamCreateWithFlags(&st0, cudaStreamNonBlocking);
         cudaGraph_t g = nullptr;
@@ -1482,23 +1485,25 @@ int cg_autotune(cg_sim* s, int reps, double ms_out[4 * CG_MAX_VARIANTS], int cho
     s->var.diff = best[3];
     // then the graph layout: each layout's graph of kStepsPerGraph steps,
     // all reading the current state (nothing steps), replayed reps times
-    double lay_ms[2] = {0.0, 0.0};
-    for (int l = 0; l < 2; ++l) {
-        s->layout = l;
-        cudaGraphExec_t ge = nullptr;
-        cudaError_t e = capture_steps(s, s->cur, kStepsPerGraph, false, &ge, true);
-        if (e == cudaSuccess) e = cudaGraphLaunch(ge, s->stream);   // warm-up
-        if (e == cudaSuccess) e = cudaEventRecord(s->ev[0], s->stream);
-        for (int r = 0; r < reps && e == cudaSuccess; ++r) e = cudaGraphLaunch(ge, s->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(s->ev[1], s->stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(s->ev[1]);
-        float t = 0.f;
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&t, s->ev[0], s->ev[1]);
-        if (ge) cudaGraphExecDestroy(ge);
-        if (e != cudaSuccess) return cuda_fail(e, "timing a graph layout");
-        lay_ms[l] = double(t) / reps / kStepsPerGraph;
+    if (layouts_differ(s)) {
+        double lay_ms[2] = {0.0, 0.0};
+        for (int l = 0; l < 2; ++l) {
+            s->layout = l;
+            cudaGraphExec_t ge = nullptr;
+            cudaError_t e = capture_steps(s, s->cur, kStepsPerGraph, false, &ge, true);
+            if (e == cudaSuccess) e = cudaGraphLaunch(ge, s->stream);   // warm-up
+            if (e == cudaSuccess) e = cudaEventRecord(s->ev[0], s->stream);
+            for (int r = 0; r < reps && e == cudaSuccess; ++r) e = cudaGraphLaunch(ge, s->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(s->ev[1], s->stream);
+            if (e == cudaSuccess) e = cudaEventSynchronize(s->ev[1]);
+            float t = 0.f;
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&t, s->ev[0], s->ev[1]);
+            if (ge) cudaGraphExecDestroy(ge);
+            if (e != cudaSuccess) return cuda_fail(e, "timing a graph layout");
+            lay_ms[l] = double(t) / reps / kStepsPerGraph;
+        }
+        s->layout = lay_ms[1] < lay_ms[0] ? 1 : 0;
     }
-    s->layout = lay_ms[1] < lay_ms[0] ? 1 : 0;
     rc = check_device_error(s);
     if (rc != CG_OK) return rc;
     return recapture(s);

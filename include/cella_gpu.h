@@ -216,7 +216,8 @@ int cg_timed_iterate(cg_sim* sim, double ms[4]);
  * cg_autotune times every variant of every phase at least `reps` times, in
  * three rounds, on the live handle (the state is not advanced), keeps the
  * fastest per phase, then
- * picks the graph layout (cg_set_graph_layout) and re-captures the step
+ * picks the graph layout (cg_set_graph_layout) where the two differ (from
+ * side 512 on) and re-captures the step
  * graphs.  ms_out[4 * CG_MAX_VARIANTS] (phase-major:
  * [row FFT v0..v4, column v0..v4, inverse row + growth v0..v4, diffusion
  * v0..v4], -1 where a variant does not exist) and chosen[4] may be NULL. */
