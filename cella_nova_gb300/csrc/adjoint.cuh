@@ -263,6 +263,13 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // 3. Growth backward, one kernel's RB rows per CTA (RT threads):
 //    U[k] rows -> u -> ubar -> forward row FFT -> written over U[k].
 // ---------------------------------------------------------------------------
+// The sides whose growth adjoint sums chains of rows (GrowthRows); its kernel is
+// the same in every variant.
+template <int LOGN>
+constexpr bool kGrowthChained = LOGN >= 6 && LOGN <= 8;
+template <int LOGN, int V>
+constexpr int kGrowthVariant = kGrowthChained<LOGN> ? 0 : V;
+
 // The rows of a CTA.  A thread adds its values to three FP32 sums before the
 // block adds the threads' sums in FP64, so which values share a thread decides
 // the parameter gradients' rounding.  At sides 64 to 256 a thread sums CHAIN
@@ -270,7 +277,7 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 // each of the CHAIN groups.  Elsewhere a thread's rows follow from the CTA shape
 // (at 16, 32 and 512 a thread has one row's 16 values in every shape) and, from
 // 1024 on, from how the rows arrive (land_rows).
-template <int LOGN, int V, bool CHAINED = (LOGN >= 6 && LOGN <= 8)>
+template <int LOGN, int V, bool CHAINED = kGrowthChained<LOGN>>
 struct GrowthRows : Geo<LOGN, V> {
     using Row = RowsInOrder;
     __device__ __forceinline__ static int first(int block) { return block * Geo<LOGN, V>::RB; }
@@ -656,13 +663,14 @@ inline bool rows_landed(int ctas) { return ctas > 4 * 152; }
 template <int LOGN, int V>
 cudaError_t prepare_backward_variant() {
     using G = Geo<LOGN, V>;
+    constexpr int GV = kGrowthVariant<LOGN, V>;
     cudaError_t e;
     const void* fns[7] = {reinterpret_cast<const void*>(k_diffusion_bwd<LOGN, V>),
-                          reinterpret_cast<const void*>(k_growth_bwd<LOGN, V>),
+                          reinterpret_cast<const void*>(k_growth_bwd<LOGN, GV>),
                           reinterpret_cast<const void*>(k_col_conv_adj<LOGN, V>),
                           reinterpret_cast<const void*>(k_row_c2r_add<LOGN, V>),
                           reinterpret_cast<const void*>(k_col_inv<LOGN, V>),
-                          reinterpret_cast<const void*>(k_growth_bwd<LOGN, V, kMayLand<LOGN>>),
+                          reinterpret_cast<const void*>(k_growth_bwd<LOGN, GV, kMayLand<LOGN>>),
                           reinterpret_cast<const void*>(k_row_c2r_add<LOGN, V, kMayLand<LOGN>>)};
     const size_t smem[7] = {DiffBwdGeo<LOGN, V>::SMEM,
                             GrowthRows<LOGN, V>::R2C_SMEM,
@@ -705,18 +713,19 @@ cudaError_t launch_diff_bwd(const BwdArgs& a, cudaStream_t st) {
 }
 template <int LOGN, int V>
 cudaError_t launch_growth_bwd(const BwdArgs& a, cudaStream_t st) {
-    using G = GrowthRows<LOGN, V>;
+    constexpr int GV = kGrowthVariant<LOGN, V>;
+    using G = GrowthRows<LOGN, GV>;
     const dim3 grid(G::N / G::RB, a.K);
     CUtensorMap umap{};
     if constexpr (kMayLand<LOGN>) {
         if (rows_landed(grid.x * grid.y)) {
             const cudaError_t e = encode_u_map(&umap, a.U, G::N, a.K, G::RB);
             if (e != cudaSuccess) return e;
-            return launch_pdl(k_growth_bwd<LOGN, V, true>, grid, G::RT, adj_row_smem<G, true>(),
+            return launch_pdl(k_growth_bwd<LOGN, GV, true>, grid, G::RT, adj_row_smem<G, true>(),
                               st, umap, a.U, a.abar, a.tw, a.ap, a.pgrad, a.K, a.err);
         }
     }
-    return launch_pdl(k_growth_bwd<LOGN, V>, grid, G::RT, G::R2C_SMEM, st, umap, a.U, a.abar, a.tw,
+    return launch_pdl(k_growth_bwd<LOGN, GV>, grid, G::RT, G::R2C_SMEM, st, umap, a.U, a.abar, a.tw,
                       a.ap, a.pgrad, a.K, a.err);
 }
 template <int LOGN, int V>

@@ -170,6 +170,28 @@ __host__ __device__ constexpr int plan_last_radix(int L, bool remfirst, int MR =
     return r;
 }
 
+// The threads that share a transform: the whole CTA, or each warp one of its
+// own.
+struct CtaThreads {
+    __device__ __forceinline__ static int tid() { return threadIdx.x; }
+    __device__ __forceinline__ static void sync() { __syncthreads(); }
+};
+struct WarpThreads {
+    __device__ __forceinline__ static int tid() { return threadIdx.x % 32; }
+    __device__ __forceinline__ static void sync() { __syncwarp(); }
+};
+
+template <int S, int J, bool SFAST>
+__device__ __forceinline__ void item_pos(int item, int& s, int& j) {
+    if constexpr (SFAST) {
+        s = item % S;
+        j = item / S;
+    } else {
+        s = item / J;
+        j = item % J;
+    }
+}
+
 // One Stockham pass (radix R, sub-transform size NS) over S sequences of
 // length L, with T threads.  Work item `item` = (sequence s, butterfly j):
 // s = item / J, j = item % J, or with SFAST the sequence index runs fastest,
@@ -185,33 +207,6 @@ __host__ __device__ constexpr int plan_last_radix(int L, bool remfirst, int MR =
 //   twp : this pass's table (tw_offset layout).
 //   ld(s, i, it, q)         -> float2
 //   st(s, i, v, it, q)      (it, q) name the register slot of the value.
-// The threads that share a transform: the whole CTA, or groups of GT
-// consecutive threads that each run a transform of their own (barrier g + 1
-// for group g, or the warp's own where a group is one).
-struct CtaThreads {
-    __device__ __forceinline__ static int tid() { return threadIdx.x; }
-    __device__ __forceinline__ static void sync() { __syncthreads(); }
-};
-template <int GT>
-struct GroupThreads {
-    __device__ __forceinline__ static int tid() { return threadIdx.x % GT; }
-    __device__ __forceinline__ static void sync() {
-        if constexpr (GT == 32) __syncwarp();
-        else asm volatile("bar.sync %0, %1;" ::"r"(threadIdx.x / GT + 1), "n"(GT) : "memory");
-    }
-};
-
-template <int S, int J, bool SFAST>
-__device__ __forceinline__ void item_pos(int item, int& s, int& j) {
-    if constexpr (SFAST) {
-        s = item % S;
-        j = item / S;
-    } else {
-        s = item / J;
-        j = item % J;
-    }
-}
-
 template <int L, int R, int NS, bool INV, int T, int S, bool SFAST = false, bool MIDBAR = true,
           class PAR = CtaThreads, class LD, class ST>
 __device__ __forceinline__ void stockham_pass(LD& ld, ST& st, const float2* __restrict__ twp) {

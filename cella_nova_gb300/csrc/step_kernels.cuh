@@ -774,10 +774,10 @@ __global__ void __launch_bounds__(C2RShape<LOGN, V>::RT, C2RShape<LOGN, V>::MINB
 
 // ---------------------------------------------------------------------------
 // The same at small sides with the kernels of the channel side by side: group
-// g of GT threads transforms kernel g, then g + the number of groups, ...,
+// g, a warp, transforms kernel g, then g + the number of groups, ...,
 // and leaves the bump's values e in shared memory; the whole CTA then adds
 // w e in increasing k (the order and the bits of row_c2r_growth_body) and
-// writes A.  One CTA of 32 or 64 threads with three kernels one after another
+// writes A.  One warp with three kernels one after another
 // is a chain of three transforms on an SM that has nothing else to do:
 // 4.4 -> 3.7 us at 256^2 with C=3, K=9.  At 512^2
 // the CTAs of row_c2r_growth_body already fill the GPU and win (5.7 against
@@ -789,6 +789,7 @@ template <int LOGN>
 struct C2RGroups : Geo<LOGN, 0> {
     using G = Geo<LOGN, 0>;
     static constexpr int GT = G::RT;
+    static_assert(GT == 32, "a group is a warp");
     static constexpr int PITCH = G::C2R_LAND + G::C2R_TILE;   // float2 per group
     static constexpr size_t SMEM = size_t(PITCH) * sizeof(float2);
     static_assert(SMEM % 128 == 0, "tensor-copy destination alignment");
@@ -800,7 +801,7 @@ __global__ void __launch_bounds__(C2RGroups<LOGN>::GT* kMaxGroups)
                      const float2* __restrict__ tw, const __grid_constant__ KernelGroups groups,
                      const GrowthParams* __restrict__ gpp, float temp, int* err, int cbase) {
     using G = C2RGroups<LOGN>;
-    using PAR = GroupThreads<G::GT>;
+    using PAR = WarpThreads;
     constexpr int N = G::N, M = G::M, RB = G::RB, GT = G::GT;
     constexpr int RL = last_radix(M, G::ROW_MR), JL = M / RL, ITEMS = RB * JL;
     constexpr int SLOTS = RB * M;   // pixel pairs of the CTA's rows
