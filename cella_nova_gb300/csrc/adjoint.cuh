@@ -658,7 +658,7 @@ constexpr size_t adj_row_smem() {
 // sides from 1024 on, and more CTAs than the four per SM that fit.
 template <int LOGN>
 constexpr bool kMayLand = LOGN > kMaxSmallLogN;
-inline bool rows_landed(int ctas) { return ctas > 4 * 152; }
+inline bool rows_landed(int ctas, int sms) { return ctas > 4 * sms; }
 
 template <int LOGN, int V>
 cudaError_t prepare_backward_variant() {
@@ -718,7 +718,7 @@ cudaError_t launch_growth_bwd(const BwdArgs& a, cudaStream_t st) {
     const dim3 grid(G::N / G::RB, a.K);
     CUtensorMap umap{};
     if constexpr (kMayLand<LOGN>) {
-        if (rows_landed(grid.x * grid.y)) {
+        if (rows_landed(grid.x * grid.y, a.sms)) {
             const cudaError_t e = encode_u_map(&umap, a.U, G::N, a.K, G::RB);
             if (e != cudaSuccess) return e;
             return launch_pdl(k_growth_bwd<LOGN, GV, true>, grid, G::RT, adj_row_smem<G, true>(),
@@ -742,7 +742,7 @@ cudaError_t launch_c2r_add(const BwdArgs& a, cudaStream_t st) {
     const float2* src = a.rowspec;
     CUtensorMap smap{};
     if constexpr (kMayLand<LOGN>) {
-        if (rows_landed(grid.x * grid.y)) {
+        if (rows_landed(grid.x * grid.y, a.sms)) {
             const cudaError_t e = encode_u_map(&smap, src, G::N, a.C, G::RB);
             if (e != cudaSuccess) return e;
             return launch_pdl(k_row_c2r_add<LOGN, V, true>, grid, G::RT, adj_row_smem<G, true>(),
@@ -769,6 +769,7 @@ cudaError_t launch_backward(const BwdArgs& a, cudaStream_t st) {
     f.tw = a.tw;
     f.udbg = nullptr;
     f.err = a.err;
+    f.sms = a.sms;
     f.groups = a.groups;
     f.gp = a.gp;
     f.var = a.var;
@@ -796,7 +797,7 @@ cudaError_t launch_backward(const BwdArgs& a, cudaStream_t st) {
 // (kgrad is transformed in place).
 template <int LOGN>
 cudaError_t launch_kgrad_final(float2* kgrad, float* hbar, int K, const float2* tw,
-                               int* err, cudaStream_t st) {
+                               int sms, int* err, cudaStream_t st) {
     using G = Geo<LOGN>;
     k_col_inv<LOGN, 0><<<dim3(G::M / G::TW, K), G::CT, size_t(G::TW) * G::CP * sizeof(float2), st>>>(
         kgrad, tw);
@@ -805,7 +806,7 @@ cudaError_t launch_kgrad_final(float2* kgrad, float* hbar, int K, const float2* 
     CUtensorMap smap{};
     bool landed = false;
     if constexpr (kMayLand<LOGN>) {
-        landed = rows_landed(grid.x * grid.y);
+        landed = rows_landed(grid.x * grid.y, sms);
         if (landed) {
             const cudaError_t e = encode_u_map(&smap, kgrad, G::N, K, G::RB);
             if (e != cudaSuccess) return e;

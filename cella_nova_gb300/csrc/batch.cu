@@ -277,7 +277,7 @@ struct cg_batch {
     // with the first step
     bool graphs_ready = false;
     int cur = 0;
-    int device = 0;
+    int device = 0, sms = 0;
     cudaGraphExec_t graph[2][2] = {};   // kBatchGraphSteps[i] steps, per parity
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     size_t max_px = 0;
@@ -379,6 +379,7 @@ StepArgs world_step_args(const cg_batch* b, int w, int parity, const Variants& v
     a.groups = W.groups;
     a.gp = &b->d_worlds[w].gp;   // the descriptor's copy, in device memory
     a.var = var;
+    a.sms = b->sms;
     return a;
 }
 
@@ -744,9 +745,8 @@ int cg_batch_create(int n_worlds, const int* n, const int* C, const int* K, cons
                        cudaMemcpyHostToDevice),
             "uploading world descriptors");
     // size classes, largest first; per class and phase a work list
-    int sms = 0;
     if (rc == CG_OK)
-        chk(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device), "attr");
+        chk(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device), "attr");
     for (int logn = kBatchMaxLogN; logn >= kBatchMinLogN && rc == CG_OK; --logn) {
         bool present = false;
         for (const auto& W : b->worlds) present = present || W.logn == logn;
@@ -794,7 +794,7 @@ int cg_batch_create(int n_worlds, const int* n, const int* C, const int* K, cons
                 chk(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pv.fn, pv.threads,
                                                                   pv.smem),
                     "occupancy");
-                sc.grid[p][v] = std::max(1, std::min(per_sm * sms, std::max(1, sc.count[p][v])));
+                sc.grid[p][v] = std::max(1, std::min(per_sm * b->sms, std::max(1, sc.count[p][v])));
             }
         b->classes.push_back(sc);
     }

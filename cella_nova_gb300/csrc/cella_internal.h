@@ -78,6 +78,7 @@ struct StepArgs {
     KernelGroups groups;
     const GrowthParams* gp;   // device-resident: updated without re-capturing graphs
     Variants var;
+    int sms;   // the device's SMs
 };
 
 // While one lives, this thread's calls may capture, instantiate and destroy
@@ -134,6 +135,7 @@ struct BwdArgs {
     // and A already hold them (a cached forward step)
     bool recompute;
     Variants var;   // CTA shapes (the forward phases' tuned variants)
+    int sms;        // the device's SMs
 };
 
 // Ring-kernel descriptors for the on-GPU kernel builder (kernels_common.cu).
@@ -171,7 +173,7 @@ typedef cudaError_t (*launch_step_channel_fn)(const StepArgs&, int phases, int c
 typedef cudaError_t (*kspec_cols_fn)(const float2* rows, float2* kspec, const float2* tw,
                                       const double* zsum, int K, cudaStream_t);
 typedef cudaError_t (*kgrad_final_fn)(float2* kgrad, float* hbar, int K, const float2* tw,
-                                      int* err, cudaStream_t);
+                                      int sms, int* err, cudaStream_t);
 
 struct SizeOps {
     launch_step_fn step;

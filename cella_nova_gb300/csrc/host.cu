@@ -224,7 +224,7 @@ struct cg_sim {
     std::vector<uint32_t> c0, c1;
     std::vector<float> mu, sigma, w;
     const SizeOps* ops = nullptr;
-    int device = 0;
+    int device = 0, sms = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     float* state[2] = {nullptr, nullptr};
@@ -294,6 +294,7 @@ struct cg_sim {
         a.groups = groups;
         a.gp = &dparams->gp;
         a.var = var;
+        a.sms = sms;
         return a;
     }
 };
@@ -627,6 +628,7 @@ BwdArgs bwd_args(cg_sim* s, const float* x, const float* ybar, float* xbar, doub
     a.ap = &s->dparams->ap;
     a.recompute = true;
     a.var = s->var;
+    a.sms = s->sms;
     return a;
 }
 
@@ -691,6 +693,9 @@ int cg_create(int n, int C, int K, const uint32_t* c0, const uint32_t* c1, const
         return rc == CG_OK;
     };
     chk(cudaGetDevice(&s->device), "cudaGetDevice");
+    if (rc == CG_OK)
+        chk(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device),
+            "cudaDeviceGetAttribute");
     if (rc == CG_OK) {
         if (stream) {
             s->stream = static_cast<cudaStream_t>(stream);
@@ -1301,8 +1306,8 @@ int cg_kernel_grad_spatial(cg_sim* s, float* kgrad, float* hbar) {
     if (!aligned16(kgrad) || !aligned16(hbar)) return misaligned("cg_kernel_grad_spatial");
     int rc = ensure_backward(s);
     if (rc != CG_OK) return rc;
-    CG_CHECK(s->ops->kgrad_final(reinterpret_cast<float2*>(kgrad), hbar, s->K, s->tw, s->err,
-                                 s->stream),
+    CG_CHECK(s->ops->kgrad_final(reinterpret_cast<float2*>(kgrad), hbar, s->K, s->tw, s->sms,
+                                 s->err, s->stream),
              "finishing the kernel gradient");
     return CG_OK;
 }

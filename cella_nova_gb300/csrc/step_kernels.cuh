@@ -410,10 +410,11 @@ __device__ __forceinline__ bool col_conv_body(const float2* __restrict__ rowspec
     constexpr uint32_t kKernelBytes = KRE ? uint32_t(TW) * N * sizeof(float) : kTileBytes;
     const uint32_t q0 = phase;
     auto buffer = [&](uint32_t q) { return KS + (NBUF == 2 ? (q & 1u) * (TW * N) : 0); };
-    // From side 1024 on a step streams more than L2 holds: the row spectra are
-    // dead once read and the kernel spectra come round a whole step later, so
-    // both leave L2 first and U, A and the state stay longer (2048^2, C=3,
-    // K=9: 151 -> 148 us per step; C=1, K=1: 42.4 -> 40.7 us).
+    // From side 1024 on the row spectra, dead once read, and the kernel spectra,
+    // which come round a whole step later, leave L2 first, so that U, A and the
+    // state stay longer (2048^2, C=3, K=9: 151 -> 148 us per step; C=1, K=1:
+    // 42.4 -> 41.1 us).  A step whose buffers fit L2 loses nothing by it: 1024^2
+    // C=2, K=4 30.8 -> 30.3 us, C=1, K=1 19.5 us either way.
     auto copy_tile = [&](float2* dst, const void* src, uint32_t bytes, uint64_t* bar) {
         if constexpr (G::SMALL) bulk_g2s(dst, src, bytes, bar);
         else bulk_g2s_once(dst, src, bytes, bar);
@@ -1642,21 +1643,18 @@ cudaError_t launch_r2c(const StepArgs& a, int c_lo, int nc, cudaStream_t st) {
     constexpr int NB = (1 << LOGN) / R::RB;
     dim3 grid(NB, nc);
     if constexpr (R::STREAM) {   // persistent: the CTAs that fit at once
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_row_r2c<LOGN, V>, R::RT,
-                                                              R::SMEM);
+        int per_sm = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, k_row_r2c<LOGN, V>, R::RT, R::SMEM);
         if (e != cudaSuccess) return e;
-        const int ctas = (per_sm > 0 ? per_sm : 1) * sms;
+        const int ctas = (per_sm > 0 ? per_sm : 1) * a.sms;
         grid = dim3(NB * nc < ctas ? NB * nc : ctas, 1);
     }
     return launch_pdl(k_row_r2c<LOGN, V>, grid, R::RT, R::SMEM, st, a.x_in, a.rowspec, a.tw, c_lo,
                       nc, a.err);
 }
-// CTAs of the column pass that a small world's launch may fill the GPU with.
-constexpr int kSmallPlaces = 152 * 4;
+// CTAs per SM that a small world's column pass may fill the GPU with.
+constexpr int kSmallPlacesPerSm = 4;
 template <int LOGN, int V>
 cudaError_t launch_col(const StepArgs& a, int c_lo, int nc, cudaStream_t st) {
     using G = Geo<LOGN, V>;
@@ -1667,7 +1665,7 @@ cudaError_t launch_col(const StepArgs& a, int c_lo, int nc, cudaStream_t st) {
         int most = 1;
         for (int c = c_lo; c < c_lo + nc; ++c)
             most = a.groups.in_count[c] > most ? a.groups.in_count[c] : most;
-        const int places = kSmallPlaces / (G::M / G::TW * a.C);
+        const int places = kSmallPlacesPerSm * a.sms / (G::M / G::TW * a.C);
         grid.z = places < 1 ? 1 : (places < most ? places : most);
     }
     if (a.kre)
