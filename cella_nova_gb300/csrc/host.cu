@@ -486,10 +486,12 @@ int capture_graph(cg_sim* s, int i, int p) {
     return e == cudaSuccess ? CG_OK : cuda_fail(e, "capturing a step graph");
 }
 
-// The step graphs that are not there yet.
+// The step graphs that are not there yet, parity by parity: in the other order
+// a 64^2 world's single steps took 12.9 instead of 12.7 us where several worlds
+// are stepped in turn, 512^2 with C=4, K=11 187.6 instead of 186.2 us for five.
 int capture_missing(cg_sim* s) {
-    for (int i = 0; i < kGraphs; ++i)
-        for (int p = 0; p < 2; ++p)
+    for (int p = 0; p < 2; ++p)
+        for (int i = 0; i < kGraphs; ++i)
             if (!s->graph[i][p]) {
                 const int rc = capture_graph(s, i, p);
                 if (rc != CG_OK) return rc;
@@ -501,13 +503,13 @@ int capture_missing(cg_sim* s) {
 // where a capture fails).
 int recapture(cg_sim* s) {
     bool had[kGraphs][2];
-    for (int i = 0; i < kGraphs; ++i)
-        for (int p = 0; p < 2; ++p) {
+    for (int p = 0; p < 2; ++p)
+        for (int i = 0; i < kGraphs; ++i) {
             had[i][p] = s->graph[i][p] != nullptr;
             drop_graph(s, i, p);
         }
-    for (int i = 0; i < kGraphs; ++i)
-        for (int p = 0; p < 2; ++p)
+    for (int p = 0; p < 2; ++p)
+        for (int i = 0; i < kGraphs; ++i)
             if (had[i][p]) {
                 const int rc = capture_graph(s, i, p);
                 if (rc != CG_OK) return rc;
