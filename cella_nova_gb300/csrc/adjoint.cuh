@@ -186,8 +186,10 @@ __device__ __forceinline__ void gather_rows(const float2* __restrict__ src, floa
 // gradient pass at 2048^2, C=2, K=4, 8 steps, 4485 -> 4133 us, at 1024^2, C=3,
 // K=9, 16 steps, 4197 -> 4127 us; with one channel and kernel at 1024^2 it
 // would take 1588 instead of 1544 us.  `plane` is the tile's plane of [M][N] in
-// the map.  Issue and wait; false (and *err) on
-// a bounded wait that timed out, for every thread alike.
+// the map.  Issue and wait; false (and *err) on a bounded wait that timed out,
+// for every thread alike.  The values are those of gather_rows, but the row
+// index runs fastest over the threads, so the growth adjoint's parameter sums
+// are grouped (and rounded) in another way; its other results have the same bits.
 template <class G>
 __device__ __forceinline__ bool land_rows(const CUtensorMap* map, int plane, int y0, float2* land,
                                           uint64_t* bar, int* err) {

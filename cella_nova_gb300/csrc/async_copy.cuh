@@ -143,8 +143,11 @@ __device__ __forceinline__ void cp_async_wait() {
 // and its memory operations are visible (a no-op for a kernel launched
 // without the attribute), and pdl_launch_dependents lets the next such
 // kernel start launching its CTAs, which then wait in their own pdl_wait.
-// The step kernels call both before touching global memory, so the overlap
-// covers only launch latency and the last wave's tail.
+// The step kernels call both before they touch what a kernel before them in
+// the stream writes, so the overlap covers launch latency, the last wave's
+// tail and, at small sides, the twiddles and kernel spectra: those were
+// written at least two kernels earlier, and the kernel in between started only
+// after its own wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

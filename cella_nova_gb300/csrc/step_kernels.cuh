@@ -58,8 +58,8 @@ struct Geo {
     // RB = 2 (2 rows x 8 columns).
     //
     // From side 1024 on the CTAs of 128 threads (V=0) won the inverse row
-    // pass: 57.5 against 65.7 and 87.1 us at 2048^2 with C=3, K=9, and 17.0
-    // against 19.2 and 31.1 us at 1024^2.  Up to side 512 a whole world is
+    // pass: 56.0 against 65.4 and 89.0 us at 2048^2 with C=3, K=9, and 16.4
+    // against 19.5 and 32.2 us at 1024^2.  Up to side 512 a whole world is
     // less work than the GPU has places for, so what counts is the number of
     // CTAs and the length of each one's chain: 4, 8 or 16 rows per CTA, a
     // thread per radix-16 butterfly, and at least a warp (at 256^2 4.6 us
@@ -93,8 +93,8 @@ struct Geo {
     // Column kernel: TW columns per CTA, CT threads (one per butterfly of a
     // radix-16 pass); a padded work buffer and an unpadded staging tile that
     // bulk copies fill.  From side 1024 on TW = 2048/N and 128 threads with
-    // V=0 (2048^2: 56.7 against 68.4 and 84.3 us; 1024^2: 17.0 against 19.5
-    // and 26.9 us); up to side 512 4, 2 or 8 columns (256^2: 2.9 us, and
+    // V=0 (2048^2: 56.3 against 66.2 and 90.2 us; 1024^2: 17.9 against 19.5
+    // and 28.5 us); up to side 512 4, 2 or 8 columns (256^2: 2.9 us, and
     // 7.8 us with 16 columns and 256 threads).
     // CVS: the CTA shape of the column pass (V=3 takes V=0's, V=4 V=1's);
     // COL_SWAP: the remainder-first plan forward, the greedy plan inverse.
@@ -778,11 +778,10 @@ __global__ void __launch_bounds__(C2RShape<LOGN, V>::RT, C2RShape<LOGN, V>::MINB
 // g, a warp, transforms kernel g, then g + the number of groups, ...,
 // and leaves the bump's values e in shared memory; the whole CTA then adds
 // w e in increasing k (the order and the bits of row_c2r_growth_body) and
-// writes A.  One warp with three kernels one after another
-// is a chain of three transforms on an SM that has nothing else to do:
-// 4.4 -> 3.7 us at 256^2 with C=3, K=9.  At 512^2
-// the CTAs of row_c2r_growth_body already fill the GPU and win (5.7 against
-// 6.1 us).
+// writes A.  One warp with three kernels one after another is a chain of three
+// transforms on an SM that has nothing else to do: 4.4 -> 3.7 us at 256^2 with
+// C=3, K=9.  At 512^2 the CTAs of row_c2r_growth_body already fill the GPU and
+// win (5.7 against 6.1 us).
 // grid (N/RB, C), block GT * groups.
 // ---------------------------------------------------------------------------
 constexpr int kMaxGroups = 4, kMaxGroupsLogN = 8;
@@ -1216,7 +1215,8 @@ __device__ __forceinline__ void diffusion_pair_body(const float* __restrict__ A,
 // registers (six CTAs per SM) it ran at 35.0 us at 2048^2, C=3, in 16-row
 // strips and 39.2 us in 8-row strips (151 MB in and out); with three rows ahead
 // at 123 registers (four CTAs) at 31.3 and 33.5 us.  Two rows at 96 registers:
-// 34.3 and 33.4 us; four rows: 30.8 and 34.1 us.
+// 34.3 and 33.4 us; four rows: 30.8 and 34.1 us.  (All before the L2 requests of
+// `ahead`, with which they take 35.9 and 32.9 us.)
 template <int LOGN, int STRIP = 16>
 struct DiffGeoReg {
     static constexpr int N = 1 << LOGN;
@@ -1347,9 +1347,9 @@ __device__ __forceinline__ void diffusion_reg_body(const float* __restrict__ A,
 // strips, 2 the column-pair body, 0 the shared-memory tile body up to side
 // 512 (at 256^2 2.4 us, against 6.6 and 4.0 us for the strips, whose rows
 // wait for their loads one after another) and the 8-row strips from 1024 on
-// (1024^2, C=3: 7.9 us, 9.2 us in 16 rows; 2048^2, C=1: both 9.1 us; C=3: 33.5
-// against 31.3 us alone, but 148.2 against 149.5 us for the whole step).  All
-// give the same bits.  TX x TY is the tile of one CTA (one work item).
+// (C=3, rows asked into L2 ahead: 32.9 us at 2048^2 and 9.0 us at 1024^2,
+// against 35.9 and 10.2 us in 16 rows; the whole step 149.2 against 150.4 us
+// and 45.8 against 48.3 us).  All give the same bits.  TX x TY is the tile of one CTA (one work item).
 constexpr int kDiffVariants = 4;
 template <int LOGN, int V,
           int KIND = V == 2 ? 2 : (V == 1 || V == 3 || LOGN > kMaxSmallLogN) ? 1 : 0>

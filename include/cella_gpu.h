@@ -201,8 +201,7 @@ int cg_timed_iterate(cg_sim* sim, double ms[4]);
  *        the grid side.  From side 1024 on the forward row FFT's variant 2
  *        is variant 1's tile in a persistent grid whose CTAs bring each
  *        block of rows in with one bulk copy, the next block's during the
- *        current one's transform, and diffusion's variant 0 takes 16- or
- *        8-row strips (variant 1 or 3) by the world's size.
+ *        current one's transform, and diffusion's variant 0 is variant 3.
  *   3    for diffusion, at every grid side: variant 1's register tiles in
  *        strips of 8 rows instead of 16; bit-identical results.
  *   3, 4 FFT plans, for the row and column phases at grid sides >= 512:
@@ -215,10 +214,11 @@ int cg_timed_iterate(cg_sim* sim, double ms[4]);
  * Diffusion has variants 0-3; the other phases below side 512 have 0-2.
  * cg_autotune times every variant of every phase at least `reps` times, in
  * three rounds, on the live handle (the state is not advanced), keeps the
- * fastest per phase, then
- * picks the graph layout (cg_set_graph_layout) where the two differ (from
- * side 512 on) and re-captures the step
- * graphs.  ms_out[4 * CG_MAX_VARIANTS] (phase-major:
+ * fastest per phase, then picks the graph layout (cg_set_graph_layout) where
+ * the two differ (from side 512 on) and re-captures the step graphs.  A phase
+ * is timed alone: between the steps of a chain up to side 512 the diffusion and
+ * the next forward row pass are one kernel without variants, which forward row
+ * variants 3 and 4 do without.  ms_out[4 * CG_MAX_VARIANTS] (phase-major:
  * [row FFT v0..v4, column v0..v4, inverse row + growth v0..v4, diffusion
  * v0..v4], -1 where a variant does not exist) and chosen[4] may be NULL. */
 #define CG_MAX_VARIANTS 5
