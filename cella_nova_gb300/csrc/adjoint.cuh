@@ -114,10 +114,18 @@ __device__ __forceinline__ void diffusion_bwd_body(const float* __restrict__ A,
                     qb = fmaf(y[(i + di) % 3][dj], av, qb);
                 }
             const Divisor by(z);
-            const float qv = by.divide(sX[r][q + 3]);
+            bool divide = false;
+            float qv = by.quotient(sX[r][q + 3], &divide);
+            float zb = by.quotient(-qb * qv, &divide);
+            float xv = by.quotient(qb, &divide);
+            if (divide) {
+                qv = sX[r][q + 3] / z;
+                zb = -qb * qv / z;
+                xv = qb / z;
+            }
             sQ[r][q] = qv;
-            sZb[r][q] = by.divide(-qb * qv);
-            if (inner && r >= 1 && r <= TY) xb[(r - 1) * N] = by.divide(qb);
+            sZb[r][q] = zb;
+            if (inner && r >= 1 && r <= TY) xb[(r - 1) * N] = xv;
         }
     }
     __syncthreads();

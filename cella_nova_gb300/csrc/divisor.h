@@ -32,13 +32,14 @@ struct Divisor {
         const float m = fabsf(d);
         plain = !(m >= 5.9604645e-8f && m <= 16777216.f);   // 2^-24, 2^24
     }
-    CG_HOST_DEVICE float divide(float x) const {
+    // The quotient, or *divide set (never cleared) where it takes a division.  A
+    // caller with several numerators tests once for all: a branch each cost a
+    // gradient pass at 1024^2 26 us of 4120, one for three nothing.
+    CG_HOST_DEVICE float quotient(float x, bool* divide) const {
         const float m = fabsf(x), q0 = x * r;
-        float q = fmaf(fmaf(-q0, z, x), r, q0);
-        if (m == 0.f) q = q0;
         // 2^-100, 2^100
-        if (plain || !((m >= 7.8886091e-31f || m == 0.f) && m <= 1.2676506e30f)) q = x / z;
-        return q;
+        *divide |= plain || !((m >= 7.8886091e-31f || m == 0.f) && m <= 1.2676506e30f);
+        return m == 0.f ? q0 : fmaf(fmaf(-q0, z, x), r, q0);
     }
 };
 

@@ -11,7 +11,11 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SHIM = """
 #include "divisor.h"
 extern "C" void divide(const float* x, const float* z, float* q, long n) {
-    for (long i = 0; i < n; ++i) q[i] = cg::Divisor(z[i]).divide(x[i]);
+    for (long i = 0; i < n; ++i) {
+        bool divide = false;
+        q[i] = cg::Divisor(z[i]).quotient(x[i], &divide);
+        if (divide) q[i] = x[i] / z[i];
+    }
 }
 """
 
